@@ -251,6 +251,9 @@ void ensure_graph(TriskModel& m, double dt) {
 }
 
 constexpr int PERSISTENT_BLOCK = 256;
+// The smallest mesh whose RK4 runs take the patches: below it (hexagon 3: 642 cells) a patch has
+// four cells and a halo of twenty, and the twelve launches a step stay.
+constexpr int64_t PATCH_RK4_MIN_CELLS = 1024;
 
 // All nsteps RK4 steps as one cooperative launch of k_rk4_persistent.
 void run_persistent(TriskModel& m, double dt, int64_t nsteps) {
@@ -278,6 +281,8 @@ void run_persistent(TriskModel& m, double dt, int64_t nsteps) {
 void run_steps(TriskModel& m, double dt, int64_t nsteps) {
   if (m.persistent) {
     run_persistent(m, dt, nsteps);
+  } else if (m.use_patches) {
+    patch_rk4(m, dt, nsteps);
   } else if (m.use_graph) {
     ensure_graph(m, dt);
     for (int64_t s = 0; s < nsteps; ++s) {
@@ -333,17 +338,18 @@ void state_out(TriskModel& m, double* y_user, const double* src) {
 }
 
 void check_flag(TriskModel& m) {
-  int flag = 0, err = 0;
-  CUDA_CHECK(cudaMemcpyAsync(&flag, m.flag, sizeof(int), cudaMemcpyDeviceToHost, m.stream));
+  int flags[2] = {0, 0}, err = 0;  // a non-finite state, a patch's wait that gave up
+  CUDA_CHECK(cudaMemcpyAsync(flags, m.flag, sizeof(flags), cudaMemcpyDeviceToHost, m.stream));
   if (m.barrier_err) CUDA_CHECK(cudaMemcpyAsync(&err, m.barrier_err, sizeof(int), cudaMemcpyDeviceToHost, m.stream));
   CUDA_CHECK(cudaStreamSynchronize(m.stream));
+  patch_check(m, flags[1]);
   if (err) {
     CUDA_CHECK(cudaMemsetAsync(m.barrier, 0, 2 * sizeof(unsigned), m.stream));
     CUDA_CHECK(cudaMemsetAsync(m.barrier_err, 0, sizeof(int), m.stream));
     CUDA_CHECK(cudaStreamSynchronize(m.stream));
     throw Error(TRISK_ERR_TIMEOUT, "a grid-barrier wait of the one-launch RK4 step gave up");
   }
-  if (flag) {
+  if (flags[0]) {
     CUDA_CHECK(cudaMemsetAsync(m.flag, 0, sizeof(int), m.stream));
     throw Error(TRISK_ERR_NONFINITE, "the state became non-finite");
   }
@@ -747,10 +753,10 @@ void finish_create(TriskModel& m, const Coefficients& C, const std::vector<V3>* 
   m.st = m.alloc<double>(m.N);
   m.stage = m.alloc<double>(m.N);
   m.dy = m.alloc<double>(m.N);
-  m.flag = m.alloc<int>(1);
+  m.flag = m.alloc<int>(2);
   m.scalars = m.alloc<double>(4);
   m.partials = m.alloc<double>(cdiv(std::max(m.nc, m.nv), RED_BLOCK * RED_PER_THREAD) + 1);
-  CUDA_CHECK(cudaMemset(m.flag, 0, sizeof(int)));
+  CUDA_CHECK(cudaMemset(m.flag, 0, 2 * sizeof(int)));
   CUDA_CHECK(cudaMemset(m.W.K, 0, m.nc * sizeof(double)));
   // state permutation: internal state index -> file index and back
   std::vector<int32_t> n2o(m.N), o2n(m.N);
@@ -764,6 +770,8 @@ void finish_create(TriskModel& m, const Coefficients& C, const std::vector<V3>* 
   CUDA_CHECK(cudaMemcpy(m.state_o2n, o2n.data(), m.N * sizeof(int32_t), cudaMemcpyHostToDevice));
   CUDA_CHECK(cudaMemcpy(m.vertex_o2n, m.vert_o2n.data(), m.nv * sizeof(int32_t), cudaMemcpyHostToDevice));
   m.C = C;
+  choose_patches(m);
+  m.use_patches = m.patches.runs && m.use_graph && !(cfg && cfg->block) && m.nc >= PATCH_RK4_MIN_CELLS;
   CUDA_CHECK(cudaDeviceSynchronize());
 }
 
@@ -955,14 +963,25 @@ int trisk_tendency(TriskModel* model, const double* y, double* dy) {
   TriskModel& m = *checked(model);
   if (!y || !dy) throw Error(TRISK_ERR_ARGUMENT, "NULL state");
   DeviceGuard guard(m.device);
-  state_in(m, y, m.y);
-  DevStage S{};
-  S.u = m.y;
-  S.h = m.y + m.ne;
-  S.dy = m.dy;
-  S.flag = m.flag;
-  enqueue_tendency(m, S, EPI_TENDENCY);
-  state_out(m, dy, m.dy);
+  const bool apart = y + m.N <= dy || dy + m.N <= y;
+  if (m.patches.n && apart && is_device_pointer(y) && is_device_pointer(dy)) {
+    // one launch, straight from the caller's state to the caller's tendency
+    order_after_caller(m.stream, m.caller_ev);
+    patch_tendency(m, y, dy, m.identity ? nullptr : m.state_n2o);
+  } else {
+    state_in(m, y, m.y);
+    if (m.patches.n) {
+      patch_tendency(m, m.y, m.dy, nullptr);
+    } else {
+      DevStage S{};
+      S.u = m.y;
+      S.h = m.y + m.ne;
+      S.dy = m.dy;
+      S.flag = m.flag;
+      enqueue_tendency(m, S, EPI_TENDENCY);
+    }
+    state_out(m, dy, m.dy);
+  }
   CUDA_CHECK(cudaStreamSynchronize(m.stream));
   TRISK_API_END
 }
@@ -1105,6 +1124,7 @@ int trisk_autotune(TriskModel* model, double* y, double dt, int32_t steps, doubl
   // the state is restored from the caller's copy before each trial. A persisting window, if
   // one was set, is left off.
   m.persistent = false;
+  m.use_patches = false;
   static const int choices[] = {64, 128, 256};
   static const int keep_mb[] = {0, 8, 16, 24, 32, 40, 48, 64};
   cudaEvent_t e0, e1;
@@ -1177,9 +1197,18 @@ int trisk_autotune(TriskModel* model, double* y, double dt, int32_t steps, doubl
       m.persistent = false;  // no cooperative launch: keep the launches
     }
   }
+  // the patches
+  bool use_patches = false;
+  if (m.patches.runs && m.use_graph) {
+    m.use_patches = true;
+    const double before = best_t;
+    trial(best[0], best[1], best[2], best_keep);  // the blocks and the prefix do not apply to them
+    use_patches = best_t < before;
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  m.persistent = use_persistent;
+  m.persistent = use_persistent && !use_patches;
+  m.use_patches = use_patches;
   for (int p = 0; p < 3; ++p) m.block[p] = best[p];
   m.l2_keep_bytes = best_keep;
   m.l2_window = false;
@@ -1213,6 +1242,7 @@ int trisk_model_set_block(TriskModel* model, const int32_t block[3]) {
   DeviceGuard guard(m.device);
   CUDA_CHECK(cudaStreamSynchronize(m.stream));
   for (int p = 0; p < 3; ++p) m.block[p] = block[p];
+  m.use_patches = false;  // the blocks are the three-launch tendency's
   if (m.graph) {  // recaptured with the new launch shapes at the next step
     cudaGraphExecDestroy(m.graph);
     m.graph = nullptr;
@@ -1260,6 +1290,7 @@ int trisk_model_set_l2_residency(TriskModel* model, int64_t bytes, int32_t windo
     if (limit < keep) CUDA_CHECK(cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, keep));
   }
   m.l2_keep_bytes = keep;
+  m.use_patches = false;  // the table block is the three-launch tendency's
   m.l2_window = win && keep > 0;
   m.T.keep_end = keep ? m.table_base + keep : nullptr;
   if (m.graph) {  // recaptured with the new table pointers and launch attributes

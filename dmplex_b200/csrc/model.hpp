@@ -9,6 +9,7 @@
 
 #include "common.hpp"
 #include "kernels.cuh"
+#include "patch.hpp"
 
 #define CUDA_CHECK(x)                                                                          \
   do {                                                                                         \
@@ -81,6 +82,8 @@ struct TriskModel {
   int persistent_grid = 0;               // co-resident blocks of 256 threads
   unsigned* barrier = nullptr;           // arrivals, generation
   int* barrier_err = nullptr;            // a grid-barrier wait gave up
+  trisk::PatchSet patches;               // whole tendencies and RK4 runs from shared memory (patch.hpp)
+  bool use_patches = false;              // for the RK4 runs; an explicit choice of launches turns it off
   trisk::Coefficients C;  // file numbering, 0-based (kept for export)
   CoefficientExport exported;
   std::vector<int32_t> cell_n2o, edge_n2o, vert_n2o, cell_o2n, edge_o2n, vert_o2n;

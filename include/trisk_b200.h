@@ -228,11 +228,14 @@ int trisk_model_info(TriskModel* model, int32_t* pv_mode, int32_t block[3], doub
  * unchanged) for every combination of the phase block sizes {64, 128, 256}, then L2-resident
  * table prefixes of 8..64 MB (trisk_model_set_l2_residency, no window) with the best blocks,
  * then the blocks again with the best prefix, then (for meshes whose tables and vectors fit
- * half the L2) the one-launch step of trisk_model_set_persistent, and keeps the fastest in
- * the model; best_ms gets its time per step. */
+ * half the L2) the one-launch step of trisk_model_set_persistent and (for meshes whose tables
+ * fit the SMs' shared memory) the patches, and keeps the fastest in the model; best_ms gets
+ * its time per step. */
 int trisk_autotune(TriskModel* model, double* y_device, double dt, int32_t steps, double* best_ms);
 /* Sets the threads per block of the three phases (vertex, flux, tend), each a multiple of 32
- * in [64, 256], as an autotuner result found earlier (no reference counterpart). */
+ * in [64, 256], as an autotuner result found earlier (no reference counterpart). RK4 steps
+ * then run as launches of those phases, on small meshes too, which otherwise run from the
+ * SMs' shared memory in one launch per call (the same numbers bit for bit). */
 int trisk_model_set_block(TriskModel* model, const int32_t block[3]);
 /* The one-launch RK4 step (no reference counterpart): on != 0 runs the RK4 steps of
  * trisk_rk4_step(_async) as one cooperative launch whose blocks do the twelve phases of every
@@ -242,7 +245,8 @@ int trisk_model_set_block(TriskModel* model, const int32_t block[3]);
  * returns TRISK_ERR_TIMEOUT. TRISK_ERR_UNSUPPORTED without cooperative launch. */
 int trisk_model_set_persistent(TriskModel* model, int32_t on);
 int trisk_model_get_persistent(TriskModel* model, int32_t* on);
-/* L2 residency of the tables (no reference counterpart). The first `bytes` of the model's
+/* L2 residency of the tables (no reference counterpart; the three-launch phases', which RK4
+ * steps use from then on). The first `bytes` of the model's
  * packed table block (the tendency phase's tables first, then the flux phase's, then the
  * vertex phase's) are loaded with an L2 evict-last policy, so they stay in L2 from one
  * phase launch and one RK4 stage to the next instead of streaming from HBM; with window = 1

@@ -329,3 +329,38 @@ def test_config_level7_gassmann_vertex(require_gpu):
     mass0 = d.total_mass(m, y)
     d.rk4_step(y, 75.0, d.tendency, d.RK4Cache(y), m, nsteps=200)
     assert abs(d.total_mass(m, y) - mass0) / mass0 < 1e-14
+
+
+@pytest.mark.parametrize("n,pv,ke,reorder", [(0, "trisk", "mixed", True), (1, "gassmann", "cell", True),
+                                             (2, "trisk", "vertex", False), (3, "gassmann_mean", "vertex", False),
+                                             (4, "trisk", "mixed", False), (5, "gassmann", "mixed", True)])
+def test_patches_bitwise(require_gpu, n, pv, ke, reorder):
+    """The patches (whole tendencies, and from hexagon 4 whole RK4 runs, from shared memory)
+    against the oracle and the three-launch tendency, bit for bit: the smallest meshes (patches
+    of four cells, a single block), numberings that are not compact, and a run of one launch."""
+    import torch
+    from oracle.oracle import Oracle
+    si = w.si_parameters()
+    g = trisk_grid(n)
+    o = Oracle(tables(n, pv, ke, False, None, **si), threads=4)
+    m = d.TRiSKShallowWater(g, pv_flux=pv, kinetic_energy=ke, reorder=reorder, **si)
+    phases = d.TRiSKShallowWater(g, pv_flux=pv, kinetic_energy=ke, reorder=reorder, block=128, **si)
+    y = w.synthetic_state(g, seed=6)
+    yd = torch.from_numpy(y).cuda()
+    dy = torch.empty_like(yd)
+    d.tendency(dy, yd, m)
+    assert np.array_equal(dy.cpu().numpy(), o.tendency(y))
+    d.tendency(yd, yd, m)  # in place
+    assert torch.equal(yd, dy)
+    a, b, ref = y.copy(), y.copy(), y.copy()
+    dt = w.courant_dt(g, 0.1)
+    before = m.launch_count()
+    d.rk4_step(a, dt, d.tendency, d.RK4Cache(a), m, nsteps=5)
+    if n >= 4:  # one launch (and the numbering in and out)
+        assert m.launch_count() - before <= 3
+    d.rk4_step(a, dt / 2, d.tendency, d.RK4Cache(a), m, nsteps=1)
+    d.rk4_step(b, dt, d.tendency, d.RK4Cache(b), phases, nsteps=5)
+    d.rk4_step(b, dt / 2, d.tendency, d.RK4Cache(b), phases, nsteps=1)
+    o.rk4_step(ref, dt, 5)
+    o.rk4_step(ref, dt / 2, 1)
+    assert np.array_equal(a, ref) and np.array_equal(b, ref)
