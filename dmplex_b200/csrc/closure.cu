@@ -16,10 +16,11 @@
 // so no operand is ever transposed in memory.
 //
 // Inference (k_mlp_forward): a persistent grid, several CTAs per SM, 64 TMEM columns each.
-//   Z1 = X W1^T   M=128 N=64 K=32  (A = XH[:, 0:32], X padded with zeros; B = W1 K-major)
-//   H1 = gelu(Z1 + b1) -> bf16 -> XH[:, 0:64]  (over X: MMA 1 has finished reading it)
-//   Z2 = H1 W2^T  M=128 N=64 K=64  (same TMEM columns: Z1 has been read)
-//   Y  = bf16(gelu(Z2 + b2)) W3^T + b3 on the CUDA cores (N = 2)
+//   Z1 = X W1^T + b1   M=128 N=64 K=32  (A = XH[:, 0:32]: X and ones; B = W1 and b1 K-major)
+//   H1 = gelu(Z1) -> bf16 -> XH[:, 0:64]  (over X: MMA 1 has finished reading it)
+//   Z2 = H1 W2^T + b2  M=128 N=64 K=80  (same TMEM columns: Z1 has been read)
+//   H2 = gelu(Z2) -> bf16 -> XH[:, 0:64]
+//   Y  = H2 W3^T + b3  M=128 N=16 K=64  (two columns used)
 // Training (k_mlp_train): forward, backward and weight gradients of one tile per step:
 //   forward    Z1 = X W1^T       M=128 N=64 K=32   (A = HX[:, 64:96] K-major, B = W1 K-major)
 //              H1 = gelu(Z1 + b1) -> bf16 -> HX[:, 0:64]
@@ -207,8 +208,8 @@ __global__ void __launch_bounds__(TILE, 2) k_mlp_train(const __nv_bfloat16* __re
       for (int k = 0; k < 16; ++k) {
         const int j = 16 * c + k;
         const float h2 = bf(gelu(v[k] + sb2[j]));
-        y[0] += h2 * sw3[j];
-        y[1] += h2 * sw3[NH + j];
+        y[0] += h2 * sw3[2 * j];
+        y[1] += h2 * sw3[2 * j + 1];
         sH2[t * NH + j] = __float2bfloat16_rn(h2);
       }
     }
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(TILE, 2) k_mlp_train(const __nv_bfloat16* __re
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
         const int j = 16 * c + k;
-        v[k] = (dy[0] * sw3[j] + dy[1] * sw3[NH + j]) * gelu_grad(v[k] + sb2[j]);
+        v[k] = (dy[0] * sw3[2 * j] + dy[1] * sw3[2 * j + 1]) * gelu_grad(v[k] + sb2[j]);
       }
       store8(DD, t, 16 * c, HX_CHUNK, v);
       store8(DD, t, 16 * c + 8, HX_CHUNK, v + 8);

@@ -28,13 +28,16 @@ constexpr int W2_BYTES = 8 * W_CHUNK;    // 64 x 64
 // + 64 B (mbarrier, TMEM address) + H2 (128 x 64 BF16) and dY (128 x 2 FP32) for training
 constexpr int SMEM_BYTES = HX_BYTES + DD_BYTES + W1_BYTES + W2_BYTES + 64 + TILE * NH * 2 + TILE * NOUT * 4;
 constexpr uint32_t TRAIN_TMEM_COLS = 256;  // two CTAs per SM share its 512 columns
-// Inference: XH (X, then H1: 8 chunks), W1, W2 and the barrier, 64 TMEM columns; at most
-// seven CTAs fit an SM's shared memory, and seven (even eight) x 64 columns fit its TMEM, so
-// no CTA ever waits in tcgen05.alloc.
+// Inference: a chunk of ones, XH (X, then H1, then H2: 8 chunks), W1, W2, b2, W3 and the barrier, 64
+// TMEM columns; six CTAs fit an SM's shared memory, and eight x 64 columns fit its TMEM, so no CTA
+// ever waits in tcgen05.alloc.
 constexpr int XH_BYTES = 8 * HX_CHUNK;
-constexpr int FWD_SMEM_BYTES = XH_BYTES + W1_BYTES + W2_BYTES + 64;
+constexpr int B2_BYTES = 2 * W_CHUNK;  // 64 x 16
+constexpr int W3_CHUNK = 16 * 16;      // one 8-column chunk of the 16-row (two used) output weight
+constexpr int W3_BYTES = 8 * W3_CHUNK;
+constexpr int FWD_SMEM_BYTES = HX_CHUNK + XH_BYTES + W1_BYTES + W2_BYTES + B2_BYTES + W3_BYTES + 64;
 constexpr uint32_t FWD_TMEM_COLS = 64;
-static_assert(FWD_SMEM_BYTES * 7 <= 220 * 1024, "seven inference CTAs per SM");
+static_assert(FWD_SMEM_BYTES * 6 <= 220 * 1024, "six inference CTAs per SM");
 // A bounded tensor-core wait gives up after this long (the operations take microseconds).
 constexpr long long MBAR_WAIT_NS = 500000000LL;
 
@@ -124,6 +127,30 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
 
+// 32 consecutive columns
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int k = 0; k < 32; ++k) v[k] = __uint_as_float(r[k]);
+}
+// two
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, float& a, float& b) {
+  uint32_t r[2];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  a = __uint_as_float(r[0]);
+  b = __uint_as_float(r[1]);
+}
+
 __device__ __forceinline__ float tanh_approx(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -143,6 +170,53 @@ __device__ __forceinline__ float gelu_grad(float x) {
   const float t = tanh_approx(x * fmaf(GELU_C1, x2, GELU_C0));
   const float du = fmaf(3.0f * GELU_C1, x2, GELU_C0);
   return fmaf(0.5f * x * fmaf(-t, t, 1.0f), du, fmaf(0.5f, t, 0.5f));
+}
+// Two FP32 values at once (Blackwell's packed instructions, each half rounded as the scalar one):
+// half the issue slots, which the epilogues of the network run out of.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(F2 x, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 tanh2(F2 x) {
+  float a, b;
+  unpack2(x, a, b);
+  return pack2(tanh_approx(a), tanh_approx(b));
+}
+// gelu(2h) of both halves, bit for bit gelu(): x = 2h, so x/2 is h itself, and u = x (C0 + C1 x^2)
+// = h (2 C0 + 8 C1 h^2), scaled by powers of two throughout. The caller halves the weights and
+// biases that form x (exact in binary), which saves the multiplication by 1/2.
+__device__ __forceinline__ F2 gelu2_of_half(F2 h) {
+  const F2 u = mul2(h, fma2(pack2(8.0f * GELU_C1, 8.0f * GELU_C1), mul2(h, h), pack2(2.0f * GELU_C0, 2.0f * GELU_C0)));
+  return fma2(h, tanh2(u), h);
+}
+// the two halves rounded to BF16 (low half first)
+__device__ __forceinline__ uint32_t bf16x2(F2 x) {
+  float a, b;
+  unpack2(x, a, b);
+  const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&p);
 }
 __device__ __forceinline__ float bf(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
@@ -166,7 +240,8 @@ struct Status {
   int error;  // 1: a bounded tensor-core wait gave up
 };
 
-// W1 (64 x 32, inputs padded with 0) and W2 (64 x 64) as K-major B operands; biases and W3
+// W1 (64 x 32, inputs padded with 0) and W2 (64 x 64) as K-major B operands; biases and W3 (unit
+// by unit, the two outputs' weights side by side)
 __device__ __forceinline__ void load_weights(unsigned char* W1s, unsigned char* W2s, float* sb1, float* sb2,
                                              float* sw3, float* sb3, const ParamsBF16* __restrict__ wbf,
                                              const Params* __restrict__ p, int t) {
@@ -184,9 +259,31 @@ __device__ __forceinline__ void load_weights(unsigned char* W1s, unsigned char* 
     sb1[idx] = p->b1[idx];
     sb2[idx] = p->b2[idx];
   }
-  for (int idx = t; idx < NOUT * NH; idx += TILE) sw3[idx] = __bfloat162float(wbf->W3[idx]);
+  for (int idx = t; idx < NOUT * NH; idx += TILE) sw3[NOUT * (idx % NH) + idx / NH] = __bfloat162float(wbf->W3[idx]);
   if (t < NOUT) sb3[t] = p->b3[t];
 }
+
+// 8 BF16 values halved (exact in binary)
+__device__ __forceinline__ uint4 half_bf16x8(const __nv_bfloat16* p) {
+  uint4 q = *reinterpret_cast<const uint4*>(p);
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
+  const __nv_bfloat162 half = __float2bfloat162_rn(0.5f);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) h[k] = __hmul2(h[k], half);
+  return q;
+}
+// x as the sum of three BF16 values (3 x 8 significant bits: exact), in columns 0..2 of a chunk row
+__device__ __forceinline__ uint4 split_bf16(float x) {
+  const __nv_bfloat16 hi = __float2bfloat16_rn(x);
+  const float r1 = x - __bfloat162float(hi);
+  const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
+  const __nv_bfloat16 lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
+  const uint32_t h = *reinterpret_cast<const uint16_t*>(&hi), m = *reinterpret_cast<const uint16_t*>(&mid),
+                 l = *reinterpret_cast<const uint16_t*>(&lo);
+  return make_uint4(h | (m << 16), l, 0u, 0u);
+}
+// columns 0..2 of a chunk row = 1: what split_bf16's three terms are multiplied with
+__device__ __forceinline__ uint4 three_ones() { return make_uint4(0x3F803F80u, 0x3F80u, 0u, 0u); }
 
 // The bounded tensor-core waits of a CTA. wait() records a give-up in the CTA's shared abort
 // word; every thread reads that word only right after a CTA-wide barrier, so all threads
@@ -214,26 +311,33 @@ struct MmaWaits {
 };
 
 // ---- inference of one tile ------------------------------------------------------------
-// A CTA of TILE threads with XH (XH_BYTES), W1s, W2s, the mbarrier and the TMEM address slot in
-// dynamic shared memory (FWD_SMEM_BYTES), FWD_TMEM_COLS tensor-memory columns, and the biases
-// and output weights in static shared memory.
+// A CTA of TILE threads with FWD_SMEM_BYTES of dynamic shared memory and FWD_TMEM_COLS
+// tensor-memory columns. Everything a row needs of the weights reaches it through the tensor
+// cores. A value read from shared memory for every row costs the shared-memory pipe a clock a
+// warp however few bytes it is: biases and output weights, 256 values a row, kept that pipe
+// 65 % busy and the tanh unit at 64 %. So a bias is three BF16 terms (exact) against columns of
+// ones (b1 in X's padding, b2 in one more K step), and the output layer is a third MMA on H2.
 struct InferSmem {
+  unsigned char* ones;  // directly before XH: the second chunk of its K step is H1's first, against zeros
   unsigned char* XH;
   unsigned char* W1s;
   unsigned char* W2s;
+  unsigned char* B2s;
+  unsigned char* W3s;
   uint64_t* mbar;
   uint32_t* tmem_slot;
   __device__ explicit InferSmem(unsigned char* smem)
-      : XH(smem), W1s(smem + XH_BYTES), W2s(smem + XH_BYTES + W1_BYTES),
-        mbar(reinterpret_cast<uint64_t*>(smem + XH_BYTES + W1_BYTES + W2_BYTES)),
-        tmem_slot(reinterpret_cast<uint32_t*>(smem + XH_BYTES + W1_BYTES + W2_BYTES + 16)) {}
+      : ones(smem), XH(ones + HX_CHUNK), W1s(XH + XH_BYTES), W2s(W1s + W1_BYTES), B2s(W2s + W2_BYTES),
+        W3s(B2s + B2_BYTES), mbar(reinterpret_cast<uint64_t*>(W3s + W3_BYTES)),
+        tmem_slot(reinterpret_cast<uint32_t*>(W3s + W3_BYTES + 16)) {}
 };
 struct InferStatic {
-  float b1[NH], b2[NH], w3[NOUT * NH], b3[NOUT];
+  float b3[NOUT];
   int abort;
 };
 
-// Tensor memory, the mbarrier and the weights; returns the CTA's TMEM base address.
+// Tensor memory, the mbarrier and the weights (W1, W2 and their biases halved, as gelu2_of_half
+// takes them); returns the CTA's TMEM base address.
 __device__ __forceinline__ uint32_t infer_setup(const InferSmem& S, InferStatic& st, const ParamsBF16* wbf,
                                                 const Params* p) {
   const int t = threadIdx.x, warp = t >> 5;
@@ -248,7 +352,27 @@ __device__ __forceinline__ uint32_t infer_setup(const InferSmem& S, InferStatic&
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     st.abort = 0;
   }
-  load_weights(S.W1s, S.W2s, st.b1, st.b2, st.w3, st.b3, wbf, p, t);
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  *reinterpret_cast<uint4*>(S.ones + tile_off(t, 0, HX_CHUNK)) = three_ones();
+  for (int idx = t; idx < NH * 4; idx += TILE) {  // W1's inputs, then b1 in the padding
+    const int r = idx >> 2, c = idx & 3;
+    *reinterpret_cast<uint4*>(S.W1s + tile_off(r, 8 * c, W_CHUNK)) =
+        c < 3 ? half_bf16x8(wbf->W1 + r * KIN + 8 * c) : split_bf16(0.5f * p->b1[r]);
+  }
+  for (int idx = t; idx < NH * 8; idx += TILE) {
+    const int r = idx >> 3, c0 = (idx & 7) * 8;
+    *reinterpret_cast<uint4*>(S.W2s + tile_off(r, c0, W_CHUNK)) = half_bf16x8(wbf->W2 + r * NH + c0);
+  }
+  {
+    const int r = t >> 1, c = t & 1;  // 64 rows x 2 chunks
+    *reinterpret_cast<uint4*>(S.B2s + tile_off(r, 8 * c, W_CHUNK)) = c == 0 ? split_bf16(0.5f * p->b2[r]) : zero;
+  }
+  {
+    const int r = t >> 3, c = t & 7;  // 16 rows x 8 chunks
+    *reinterpret_cast<uint4*>(S.W3s + tile_off(r, 8 * c, W3_CHUNK)) =
+        r < NOUT ? *reinterpret_cast<const uint4*>(wbf->W3 + r * NH + 8 * c) : zero;
+  }
+  if (t < NOUT) st.b3[t] = p->b3[t];
   fence_async_smem();
   fence_before();
   __syncthreads();
@@ -256,18 +380,39 @@ __device__ __forceinline__ uint32_t infer_setup(const InferSmem& S, InferStatic&
   return *S.tmem_slot;
 }
 
-// Row t of the tile's features (24 BF16 values as three 16-byte chunks) into XH chunks 0..2,
-// and zeros into chunk 3 (W1's padding columns are 0 as well).
+// Row t of the tile's features (24 BF16 values as three 16-byte chunks) into XH chunks 0..2, and
+// the ones of b1's columns into chunk 3.
 __device__ __forceinline__ void infer_put_row(const InferSmem& S, const uint4 (&q)[3]) {
   const int t = threadIdx.x;
 #pragma unroll
   for (int c = 0; c < 3; ++c) *reinterpret_cast<uint4*>(S.XH + tile_off(t, 8 * c, HX_CHUNK)) = q[c];
-  *reinterpret_cast<uint4*>(S.XH + tile_off(t, 24, HX_CHUNK)) = make_uint4(0, 0, 0, 0);
+  *reinterpret_cast<uint4*>(S.XH + tile_off(t, 24, HX_CHUNK)) = three_ones();
+}
+
+// bf16(gelu(2 Z)) of this thread's row of Z (64 TMEM columns) into XH's row
+__device__ __forceinline__ void infer_activate(const InferSmem& S, uint32_t lane_base) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    float v[32];
+    tmem_ld32(lane_base + 32 * c, v);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // 8 columns, one 16-byte store
+      uint32_t h[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) h[k] = bf16x2(gelu2_of_half(pack2(v[8 * q + 2 * k], v[8 * q + 2 * k + 1])));
+      *reinterpret_cast<uint4*>(S.XH + tile_off(t, 32 * c + 8 * q, HX_CHUNK)) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+  }
 }
 
 // The network on the tile in XH (all threads call it after writing their rows): this thread's
 // two outputs; false if the CTA has given up a wait (then every thread returns false). With
-// issue = false the first tensor-core operation is left out (the bounded wait's test).
+// issue = false the first tensor-core operation is left out (the bounded wait's test). What
+// bounds it is the special-function unit (128 tanh a row at 16 a clock: 1024 clocks a tile; 67 %
+// busy by ncu) and the latency of three barrier and tensor-core round trips a tile behind it.
+// Measured on 3.9 M rows: 253 us with scalar epilogues and shared-memory biases, 205 us with
+// packed ones, 194 us in this form.
 __device__ __forceinline__ bool infer_tile(const InferSmem& S, const InferStatic& st, uint32_t tmem, MmaWaits& waits,
                                            bool issue, float& y0, float& y1) {
   const int t = threadIdx.x, warp = t >> 5;
@@ -280,67 +425,43 @@ __device__ __forceinline__ bool infer_tile(const InferSmem& S, const InferStatic
     __syncthreads();
     fence_after();
   };
-  const float4* b1v = reinterpret_cast<const float4*>(st.b1);
-  const float4* b2v = reinterpret_cast<const float4*>(st.b2);
-  const float4* w3a = reinterpret_cast<const float4*>(st.w3);
-  const float4* w3b = reinterpret_cast<const float4*>(st.w3 + NH);
   sync_for_mma();
   if (waits.aborted()) return false;
-  if (t == 0 && issue) {  // Z1 = X W1^T
+  if (t == 0 && issue) {  // Z1 = X W1^T + b1
 #pragma unroll
     for (int kk = 0; kk < 2; ++kk)
       mma_bf16(tmem, sdesc(xh + 2 * kk * HX_CHUNK, HX_CHUNK, 128), sdesc(w1 + 2 * kk * W_CHUNK, W_CHUNK, 128), ID, kk);
     mma_commit(waits.mb);
   }
   waits.wait(issue);
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {  // H1 = gelu(Z1 + b1) -> XH chunks 0..7 (MMA 1 has read X)
-    float v[16];
-    tmem_ld16(lane_base + 16 * c, v);
-#pragma unroll
-    for (int k4 = 0; k4 < 4; ++k4) {
-      const float4 b = b1v[4 * c + k4];
-      v[4 * k4 + 0] = gelu(v[4 * k4 + 0] + b.x);
-      v[4 * k4 + 1] = gelu(v[4 * k4 + 1] + b.y);
-      v[4 * k4 + 2] = gelu(v[4 * k4 + 2] + b.z);
-      v[4 * k4 + 3] = gelu(v[4 * k4 + 3] + b.w);
-    }
-    store8(S.XH, t, 16 * c, HX_CHUNK, v);
-    store8(S.XH, t, 16 * c + 8, HX_CHUNK, v + 8);
-  }
-  sync_for_mma();  // also: every thread has read Z1, which Z2 overwrites
+  infer_activate(S, lane_base);  // H1 (MMA 1 has read X)
+  sync_for_mma();                // also: every thread has read Z1, which Z2 overwrites
   if (waits.aborted()) return false;
-  if (t == 0) {  // Z2 = H1 W2^T
+  if (t == 0) {  // Z2 = H1 W2^T + b2
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
       mma_bf16(tmem, sdesc(xh + 2 * kk * HX_CHUNK, HX_CHUNK, 128), sdesc(w2 + 2 * kk * W_CHUNK, W_CHUNK, 128), ID, kk);
+    mma_bf16(tmem, sdesc(smem_u32(S.ones), HX_CHUNK, 128), sdesc(smem_u32(S.B2s), W_CHUNK, 128), ID, 1);
     mma_commit(waits.mb);
   }
   waits.wait(true);
-  y0 = st.b3[0];
-  y1 = st.b3[1];
+  infer_activate(S, lane_base);  // H2 (MMA 2 has read H1)
+  sync_for_mma();
+  if (waits.aborted()) return false;
+  if (t == 0) {  // Y = H2 W3^T
+    const uint32_t w3 = smem_u32(S.W3s);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {  // Y = bf16(gelu(Z2 + b2)) W3^T + b3, FP32 accumulation
-    float v[16];
-    tmem_ld16(lane_base + 16 * c, v);
-#pragma unroll
-    for (int k4 = 0; k4 < 4; ++k4) {
-      const float4 b = b2v[4 * c + k4], wa = w3a[4 * c + k4], wb = w3b[4 * c + k4];
-      const __nv_bfloat162 h01 = __floats2bfloat162_rn(gelu(v[4 * k4 + 0] + b.x), gelu(v[4 * k4 + 1] + b.y));
-      const __nv_bfloat162 h23 = __floats2bfloat162_rn(gelu(v[4 * k4 + 2] + b.z), gelu(v[4 * k4 + 3] + b.w));
-      const float h0 = __low2float(h01), h1 = __high2float(h01), h2 = __low2float(h23), h3 = __high2float(h23);
-      y0 += h0 * wa.x;
-      y1 += h0 * wb.x;
-      y0 += h1 * wa.y;
-      y1 += h1 * wb.y;
-      y0 += h2 * wa.z;
-      y1 += h2 * wb.z;
-      y0 += h3 * wa.w;
-      y1 += h3 * wb.w;
-    }
+    for (int kk = 0; kk < 4; ++kk)
+      mma_bf16(tmem, sdesc(xh + 2 * kk * HX_CHUNK, HX_CHUNK, 128), sdesc(w3 + 2 * kk * W3_CHUNK, W3_CHUNK, 128),
+               idesc_bf16(128, 16, 0, 0), kk);
+    mma_commit(waits.mb);
   }
+  waits.wait(true);
+  tmem_ld2(lane_base, y0, y1);
+  y0 += st.b3[0];
+  y1 += st.b3[1];
   fence_before();
-  __syncthreads();  // the next tile rewrites XH, and its MMA 1 overwrites Z2
+  __syncthreads();  // the next tile rewrites XH, and its MMA 1 overwrites Y
   fence_after();
   return !waits.aborted();
 }
