@@ -21,17 +21,25 @@
 //   Z2 = H1 W2^T + b2  M=128 N=64 K=80  (same TMEM columns: Z1 has been read)
 //   H2 = gelu(Z2) -> bf16 -> XH[:, 0:64]
 //   Y  = H2 W3^T + b3  M=128 N=16 K=64  (two columns used)
-// Training (k_mlp_train): forward, backward and weight gradients of one tile per step:
-//   forward    Z1 = X W1^T       M=128 N=64 K=32   (A = HX[:, 64:96] K-major, B = W1 K-major)
-//              H1 = gelu(Z1 + b1) -> bf16 -> HX[:, 0:64]
-//              Z2 = H1 W2^T      M=128 N=64 K=64   (A = HX[:, 0:64], B = W2 K-major)
-//              H2 = gelu(Z2 + b2);  Y = H2 W3^T + b3 on the CUDA cores (N = 2)
-//   backward   dH2 = (dY W3) * gelu'(Z2)                       CUDA cores -> DD[:, 0:64]
-//              G = dH2 W2        M=128 N=64 K=64   (A = DD[:, 0:64] K-major, B = W2 MN-major)
-//              dH1 = G * gelu'(Z1)                             -> DD[:, 64:128]
-//              DW += DD^T [H1 | X]   M=128 N=96 K=128 (A = DD MN-major, B = HX MN-major):
-//                   rows 0..63 x cols 0..63 = dW2, rows 64..127 x cols 64..87 = dW1
-//   Tensor memory: Z1 at 0, Z2 (then G) at 64, DW at 128..224 (256 columns, two CTAs per SM).
+// Training (k_mlp_train): forward, backward and weight gradients of one tile per step, every
+// product with a weight or over the rows on the tensor cores:
+//   Z1 = X W1^T + b1, H1 = gelu(Z1), gelu'(Z1) -> TMEM (over Z1)
+//   Z2 = H1 W2^T + b2, H2 = gelu(Z2), gelu'(Z2) in registers
+//   Y  = H2 W3^T (+ b3);  dY = 2 (Y - target) / n, as three BF16 terms each (exact: 24 bits)
+//   P  = dY W3           M=128 N=64 K=16   (A = dY K-major, B = W3 transposed)
+//   dH2 = P * gelu'(Z2) -> DD[:, 0:64]
+//   G  = dH2 W2          M=128 N=64 K=64   (A = DD[:, 0:64] K-major, B = W2 MN-major)
+//   dH1 = G * gelu'(Z1) -> DD[:, 64:128]
+//   DW += DD^T [H1 | X | 1]  M=128 N=96 K=128 (A = DD MN-major, B = HX MN-major): rows 0..63 x
+//         cols 0..63 = dW2, rows 64..127 x cols 64..87 = dW1, column 88 the biases
+//   DW3 += [H2 | .]^T dY     M=128 N=16 K=128 (rows 0..63 used)
+//   Tensor memory: Z1 then gelu'(Z1) at 0, Z2 then P then G at 64, DW at 128..224, Y at 224, DW3
+//   at 240 (256 columns, two CTAs per SM).
+// Every tanh is evaluated once, gelu' being kept from the forward pass. What bounds a tile is the
+// latency of its seven barrier and tensor-core round trips, two CTAs an SM hiding one another's.
+// Measured, a training step of 65536 rows (kernel, sums read back, Adam): 95 us with dW3, the
+// output layer and the biases on the CUDA cores and every tanh evaluated twice, 55 us like this; a
+// step of 1000 rows, nearly all host calls, takes 47.
 //
 // GELU is the tanh form of Hendrycks and Gimpel (2016), gelu(x) = x/2 (1 + tanh(sqrt(2/pi)
 // (x + 0.044715 x^3))), with tanh on the special-function unit (tanh.approx.f32); it is the
@@ -45,6 +53,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 #include <memory>
 
@@ -95,11 +104,11 @@ __global__ void __launch_bounds__(TILE) k_mlp_forward(const __nv_bfloat16* __res
 
 // Training accumulates the gradients of the mean squared error (1/n) sum_rows sum_k
 // (y_k - t_k)^2 into grad (FP32, zeroed by the caller) and the squared-error sum into *loss.
-// Column 88 of HX (the first padding column of the input chunk) holds 1 for valid rows, so
-// the weight-gradient MMA also returns the bias gradients: DW[j][88] = sum_rows dH2[:, j] =
-// db2[j], DW[64 + i][88] = db1[i]. W1's padded input columns are 0, so the forward product
-// ignores it.
+// Columns 88..90 of HX (the first padding columns of the input chunk) hold 1 for valid rows: they
+// carry b1 into Z1 (and, as a chunk of their own, b2 into Z2), and through the weight-gradient
+// MMA column 88 returns the bias gradients: DW[j][88] = db2[j], DW[64 + i][88] = db1[i].
 constexpr int ONES_COL = 64 + NIN;
+constexpr uint32_t TRAIN_DW = 128, TRAIN_Y = 224, TRAIN_DW3 = 240;
 
 __global__ void __launch_bounds__(TILE, 2) k_mlp_train(const __nv_bfloat16* __restrict__ X, int64_t n,
                                                        const ParamsBF16* __restrict__ wbf,
@@ -108,14 +117,17 @@ __global__ void __launch_bounds__(TILE, 2) k_mlp_train(const __nv_bfloat16* __re
                                                        float* loss, float inv_n, Status* status) {
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* HX = smem;
-  unsigned char* DD = smem + HX_BYTES;
-  unsigned char* W1s = DD + DD_BYTES;
+  unsigned char* H2 = HX + HX_BYTES;  // after HX's ones chunk, before DD: both are read across the border
+  unsigned char* DD = H2 + H2_BYTES;
+  unsigned char* DY = DD + DD_BYTES;
+  unsigned char* W1s = DY + DY_BYTES;
   unsigned char* W2s = W1s + W1_BYTES;
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(W2s + W2_BYTES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(W2s + W2_BYTES + 16);
-  __nv_bfloat16* sH2 = reinterpret_cast<__nv_bfloat16*>(W2s + W2_BYTES + 64);  // 128 x 64
-  float* sDY = reinterpret_cast<float*>(W2s + W2_BYTES + 64 + TILE * NH * 2);   // 128 x 2
-  __shared__ float sb1[NH], sb2[NH], sw3[NOUT * NH], sb3[NOUT];
+  unsigned char* B2s = W2s + W2_BYTES;
+  unsigned char* W3s = B2s + B2_BYTES;
+  unsigned char* W3t = W3s + W3_BYTES;  // 64 units x 16: W3 of output 0 three times, of output 1 three times
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(W3t + 2 * W_CHUNK);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(W3t + 2 * W_CHUNK + 16);
+  __shared__ float sb3[NOUT];
   __shared__ int s_abort;
 
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -133,189 +145,232 @@ __global__ void __launch_bounds__(TILE, 2) k_mlp_train(const __nv_bfloat16* __re
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_abort = 0;
   }
-  load_weights(W1s, W2s, sb1, sb2, sw3, sb3, wbf, p, t);
+  load_weights(W1s, W2s, B2s, W3s, wbf, p, t);
+  if (t < NH) {
+    const uint16_t* w3 = reinterpret_cast<const uint16_t*>(wbf->W3);
+    const uint32_t a = w3[t], b = w3[NH + t];
+    *reinterpret_cast<uint4*>(W3t + tile_off(t, 0, W_CHUNK)) = make_uint4(a | (a << 16), a | (b << 16), b | (b << 16), 0);
+    *reinterpret_cast<uint4*>(W3t + tile_off(t, 8, W_CHUNK)) = make_uint4(0, 0, 0, 0);
+  }
+  // H2's first chunk is b2's second K chunk (against zeros) before a tile has filled it
+  *reinterpret_cast<uint4*>(H2 + tile_off(t, 0, HX_CHUNK)) = make_uint4(0, 0, 0, 0);
+  *reinterpret_cast<uint4*>(DY + tile_off(t, 8, HX_CHUNK)) = make_uint4(0, 0, 0, 0);
+  if (t < NOUT) sb3[t] = p->b3[t];
   fence_async_smem();
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-  const uint32_t hx = smem_u32(HX), dd = smem_u32(DD), w1 = smem_u32(W1s), w2 = smem_u32(W2s);
-  const uint32_t ID_FWD = idesc_bf16(128, 64, 0, 0), ID_BWD = idesc_bf16(128, 64, 0, 1),
-                 ID_WGRAD = idesc_bf16(128, 96, 1, 1);
+  const uint32_t hx = smem_u32(HX), h2 = smem_u32(H2), dd = smem_u32(DD), dy = smem_u32(DY), w1 = smem_u32(W1s),
+                 w2 = smem_u32(W2s), b2 = smem_u32(B2s), w3 = smem_u32(W3s), w3t = smem_u32(W3t);
+  const uint32_t ID = idesc_bf16(128, 64, 0, 0), ID_G = idesc_bf16(128, 64, 0, 1), ID_DW = idesc_bf16(128, 96, 1, 1),
+                 ID_Y = idesc_bf16(128, 16, 0, 0), ID_DW3 = idesc_bf16(128, 16, 1, 1);
   MmaWaits waits(smem_u32(mbar), &s_abort);
-  bool first_wgrad = true;
-  float loss_local = 0.0f, gw3 = 0.0f, gb3 = 0.0f;  // thread t: dW3[t / 64][t % 64]; t < 2: db3[t]
+  bool first = true;
+  float loss_local = 0.0f, gb3[NOUT] = {0.0f, 0.0f};
   auto sync_for_mma = [&]() {  // shared-memory writes -> visible to the tensor core
     fence_async_smem();
     fence_before();
     __syncthreads();
     fence_after();
   };
+  auto put32 = [&](unsigned char* base, int c0, const uint32_t* q) {  // 32 BF16 columns of row t
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      *reinterpret_cast<uint4*>(base + tile_off(t, c0 + 8 * k, HX_CHUNK)) =
+          make_uint4(q[4 * k], q[4 * k + 1], q[4 * k + 2], q[4 * k + 3]);
+  };
 
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int64_t row = tile * TILE + t;
     const bool valid = row < n;
-    // X -> HX[:, 64:96]: 24 features as three 16-byte chunks, then [1 (valid rows), 0 x 7]
-    {
+    float2 want = make_float2(0.0f, 0.0f);
+    {  // X -> HX[:, 64:88], the ones of a valid row
       uint4 q[3] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
       if (valid) {
         const uint4* src = reinterpret_cast<const uint4*>(X + row * NIN);
         q[0] = src[0];
         q[1] = src[1];
         q[2] = src[2];
+        want = make_float2(target[row * NOUT], target[row * NOUT + 1]);
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) *reinterpret_cast<uint4*>(HX + tile_off(t, 64 + 8 * c, HX_CHUNK)) = q[c];
-      float ones[8] = {valid ? 1.0f : 0.0f, 0, 0, 0, 0, 0, 0, 0};
-      store8(HX, t, ONES_COL, HX_CHUNK, ones);
+      *reinterpret_cast<uint4*>(HX + tile_off(t, ONES_COL, HX_CHUNK)) = valid ? three_ones() : make_uint4(0, 0, 0, 0);
     }
     sync_for_mma();
     if (waits.aborted()) break;
-    if (t == 0) {  // Z1 = X W1^T
+    if (t == 0) {  // Z1 = X W1^T + b1
 #pragma unroll
       for (int kk = 0; kk < 2; ++kk)
-        mma_bf16(tmem + 0, sdesc(hx + (8 + 2 * kk) * HX_CHUNK, HX_CHUNK, 128),
-                 sdesc(w1 + 2 * kk * W_CHUNK, W_CHUNK, 128), ID_FWD, kk);
+        mma_bf16(tmem, sdesc(hx + (8 + 2 * kk) * HX_CHUNK, HX_CHUNK, 128), sdesc(w1 + 2 * kk * W_CHUNK, W_CHUNK, 128),
+                 ID, kk);
       mma_commit(waits.mb);
     }
     waits.wait(true);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {  // H1 = gelu(Z1 + b1) -> HX[:, 0:64]
-      float v[16];
-      tmem_ld16(lane_base + 16 * c, v);
+    for (int c = 0; c < 2; ++c) {  // H1 -> HX[:, 0:64], gelu'(Z1) over Z1
+      float v[32];
+      uint32_t q[16];
+      tmem_ld32(lane_base + 32 * c, v);
 #pragma unroll
-      for (int k = 0; k < 16; ++k) v[k] = gelu(v[k] + sb1[16 * c + k]);
-      store8(HX, t, 16 * c, HX_CHUNK, v);
-      store8(HX, t, 16 * c + 8, HX_CHUNK, v + 8);
+      for (int k = 0; k < 16; ++k) {
+        F2 g;
+        q[k] = bf16x2(gelu2_of_half(pack2(v[2 * k], v[2 * k + 1]), g));
+        unpack2(g, v[2 * k], v[2 * k + 1]);
+      }
+      put32(HX, 32 * c, q);
+      tmem_st32(lane_base + 32 * c, v);
     }
     sync_for_mma();
     if (waits.aborted()) break;
-    if (t == 0) {  // Z2 = H1 W2^T
+    if (t == 0) {  // Z2 = H1 W2^T + b2
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-        mma_bf16(tmem + 64, sdesc(hx + 2 * kk * HX_CHUNK, HX_CHUNK, 128), sdesc(w2 + 2 * kk * W_CHUNK, W_CHUNK, 128),
-                 ID_FWD, kk);
+        mma_bf16(tmem + 64, sdesc(hx + 2 * kk * HX_CHUNK, HX_CHUNK, 128), sdesc(w2 + 2 * kk * W_CHUNK, W_CHUNK, 128), ID,
+                 kk);
+      mma_bf16(tmem + 64, sdesc(hx + 11 * HX_CHUNK, HX_CHUNK, 128), sdesc(b2, W_CHUNK, 128), ID, 1);
       mma_commit(waits.mb);
     }
     waits.wait(true);
-    float y[NOUT] = {sb3[0], sb3[1]};
+    F2 grad2[NH / 2];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {  // Y = bf16(gelu(Z2 + b2)) W3^T + b3, FP32 accumulation
-      float v[16];
-      tmem_ld16(lane_base + 64 + 16 * c, v);
+    for (int c = 0; c < 2; ++c) {  // H2, gelu'(Z2)
+      float v[32];
+      uint32_t q[16];
+      tmem_ld32(lane_base + 64 + 32 * c, v);
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const int j = 16 * c + k;
-        const float h2 = bf(gelu(v[k] + sb2[j]));
-        y[0] += h2 * sw3[2 * j];
-        y[1] += h2 * sw3[2 * j + 1];
-        sH2[t * NH + j] = __float2bfloat16_rn(h2);
-      }
+      for (int k = 0; k < 16; ++k) q[k] = bf16x2(gelu2_of_half(pack2(v[2 * k], v[2 * k + 1]), grad2[16 * c + k]));
+      put32(H2, 32 * c, q);
     }
-    // ---- backward ----
-    float dy[NOUT];
-#pragma unroll
-    for (int k = 0; k < NOUT; ++k) {
-      const float diff = valid ? y[k] - target[row * NOUT + k] : 0.0f;
-      loss_local += diff * diff;
-      dy[k] = 2.0f * diff * inv_n;
-      sDY[t * NOUT + k] = dy[k];
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {  // dH2 = (dY W3) * gelu'(Z2 + b2) -> DD[:, 0:64]
-      float v[16];
-      tmem_ld16(lane_base + 64 + 16 * c, v);
-#pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const int j = 16 * c + k;
-        v[k] = (dy[0] * sw3[2 * j] + dy[1] * sw3[2 * j + 1]) * gelu_grad(v[k] + sb2[j]);
-      }
-      store8(DD, t, 16 * c, HX_CHUNK, v);
-      store8(DD, t, 16 * c + 8, HX_CHUNK, v + 8);
-    }
-    sync_for_mma();  // also publishes sH2 and sDY
+    sync_for_mma();
     if (waits.aborted()) break;
-    if (t == 0) {    // G = dH2 W2 (overwrites Z2)
+    if (t == 0) {  // Y = H2 W3^T
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-        mma_bf16(tmem + 64, sdesc(dd + 2 * kk * HX_CHUNK, HX_CHUNK, 128), sdesc(w2 + 2 * kk * 128, 128, W_CHUNK),
-                 ID_BWD, kk);
+        mma_bf16(tmem + TRAIN_Y, sdesc(h2 + 2 * kk * HX_CHUNK, HX_CHUNK, 128),
+                 sdesc(w3 + 2 * kk * W3_CHUNK, W3_CHUNK, 128), ID_Y, kk);
       mma_commit(waits.mb);
     }
-    {  // meanwhile: dW3[o][j] += sum_rows dY[:, o] H2[:, j], db3 += sum_rows dY
-      const int o = t / NH, j = t % NH;
-      float s = 0.0f;
-      for (int r = 0; r < TILE; ++r) s += sDY[r * NOUT + o] * __bfloat162float(sH2[r * NH + j]);
-      gw3 += s;
-      if (t < NOUT) {
-        float b = 0.0f;
-        for (int r = 0; r < TILE; ++r) b += sDY[r * NOUT + t];
-        gb3 += b;
-      }
+    waits.wait(true);
+    {
+      float y0, y1;
+      tmem_ld2(lane_base + TRAIN_Y, y0, y1);
+      const float e0 = valid ? y0 + sb3[0] - want.x : 0.0f, e1 = valid ? y1 + sb3[1] - want.y : 0.0f;
+      loss_local += e0 * e0;
+      loss_local += e1 * e1;
+      const float d0 = 2.0f * e0 * inv_n, d1 = 2.0f * e1 * inv_n;
+      gb3[0] += d0;
+      gb3[1] += d1;
+      const uint4 a = split_bf16(d0), b = split_bf16(d1);  // columns 0..2 and 3..5
+      *reinterpret_cast<uint4*>(DY + tile_off(t, 0, HX_CHUNK)) =
+          make_uint4(a.x, a.y | (b.x << 16), (b.x >> 16) | (b.y << 16), 0);
+    }
+    sync_for_mma();
+    if (waits.aborted()) break;
+    if (t == 0) {  // P = dY W3 (over Z2) and DW3 += [H2 | .]^T dY
+      mma_bf16(tmem + 64, sdesc(dy, HX_CHUNK, 128), sdesc(w3t, W_CHUNK, 128), ID, 0);
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)
+        mma_bf16(tmem + TRAIN_DW3, sdesc(h2 + 2 * kk * 128, 128, HX_CHUNK), sdesc(dy + 2 * kk * 128, 128, HX_CHUNK),
+                 ID_DW3, (first && kk == 0) ? 0 : 1);
+      mma_commit(waits.mb);
     }
     waits.wait(true);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {  // dH1 = G * gelu'(Z1 + b1) -> DD[:, 64:128]
-      float g[16], z[16];
-      tmem_ld16(lane_base + 64 + 16 * c, g);
-      tmem_ld16(lane_base + 16 * c, z);
+    for (int c = 0; c < 2; ++c) {  // dH2 = P * gelu'(Z2) -> DD[:, 0:64]
+      float v[32];
+      uint32_t q[16];
+      tmem_ld32(lane_base + 64 + 32 * c, v);
 #pragma unroll
-      for (int k = 0; k < 16; ++k) g[k] *= gelu_grad(z[k] + sb1[16 * c + k]);
-      store8(DD, t, 64 + 16 * c, HX_CHUNK, g);
-      store8(DD, t, 64 + 16 * c + 8, HX_CHUNK, g + 8);
+      for (int k = 0; k < 16; ++k) q[k] = bf16x2(mul2(pack2(v[2 * k], v[2 * k + 1]), grad2[16 * c + k]));
+      put32(DD, 32 * c, q);
+    }
+    sync_for_mma();
+    if (waits.aborted()) break;
+    if (t == 0) {  // G / 2 = dH2 W2 / 2 (over P; W2s holds W2 / 2)
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)
+        mma_bf16(tmem + 64, sdesc(dd + 2 * kk * HX_CHUNK, HX_CHUNK, 128), sdesc(w2 + 2 * kk * 128, 128, W_CHUNK), ID_G,
+                 kk);
+      mma_commit(waits.mb);
+    }
+    waits.wait(true);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {  // dH1 = G * gelu'(Z1) -> DD[:, 64:128]
+      float v[16], g[16];
+      uint32_t q[8];
+      tmem_ld16(lane_base + 64 + 16 * c, v);
+      tmem_ld16(lane_base + 16 * c, g);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const F2 G = pack2(v[2 * k], v[2 * k + 1]);
+        q[k] = bf16x2(mul2(add2(G, G), pack2(g[2 * k], g[2 * k + 1])));
+      }
+      *reinterpret_cast<uint4*>(DD + tile_off(t, 64 + 16 * c, HX_CHUNK)) = make_uint4(q[0], q[1], q[2], q[3]);
+      *reinterpret_cast<uint4*>(DD + tile_off(t, 72 + 16 * c, HX_CHUNK)) = make_uint4(q[4], q[5], q[6], q[7]);
     }
     sync_for_mma();
     if (waits.aborted()) break;
     if (t == 0) {  // DW += DD^T [H1 | X | 1]
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk)
-        mma_bf16(tmem + 128, sdesc(dd + 2 * kk * 128, 128, HX_CHUNK), sdesc(hx + 2 * kk * 128, 128, HX_CHUNK),
-                 ID_WGRAD, (first_wgrad && kk == 0) ? 0 : 1);
+        mma_bf16(tmem + TRAIN_DW, sdesc(dd + 2 * kk * 128, 128, HX_CHUNK), sdesc(hx + 2 * kk * 128, 128, HX_CHUNK), ID_DW,
+                 (first && kk == 0) ? 0 : 1);
       mma_commit(waits.mb);
     }
-    first_wgrad = false;
+    first = false;
     waits.wait(true);
     fence_before();
-    __syncthreads();  // the next tile rewrites HX, DD, sH2 and sDY
+    __syncthreads();  // the next tile rewrites HX, DD and dY
     fence_after();
     if (waits.aborted()) break;
   }
 
   waits.drain();
-  if (!waits.aborted() && !first_wgrad) {  // row t of DW: dW2 and db2 (t < 64) or dW1 and db1
-    float v[16];
+  auto add16 = [](float* to, const float* v) {
+#pragma unroll
+    for (int k = 0; k < 16; k += 4)
+      atomicAdd(reinterpret_cast<float4*>(to + k), make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]));
+  };
+  if (!waits.aborted() && !first) {  // row t of DW: dW2 and db2 (t < 64) or dW1 and db1
+    float v[16], u[16];
+    tmem_ld16(lane_base + TRAIN_DW + 80, v);  // columns 80..95: inputs 16..23, then the ones
     if (t < NH) {
+      atomicAdd(&grad->b2[t], v[ONES_COL - 80]);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        tmem_ld16(lane_base + 128 + 16 * c, v);
-#pragma unroll
-        for (int k = 0; k < 16; ++k) atomicAdd(&grad->W2[t * NH + 16 * c + k], v[k]);
+        tmem_ld16(lane_base + TRAIN_DW + 16 * c, u);
+        add16(&grad->W2[t * NH + 16 * c], u);
       }
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        tmem_ld16(lane_base + 128 + 64 + 16 * c, v);
-        if (c == 1) atomicAdd(&grad->b2[t], v[ONES_COL - 64 - 16]);
-      }
+      tmem_ld16(lane_base + TRAIN_DW3, u);  // dW3[o][t]: the sums over dY's three terms
+      atomicAdd(&grad->W3[t], u[0] + (u[1] + u[2]));
+      atomicAdd(&grad->W3[NH + t], u[3] + (u[4] + u[5]));
     } else {
+      float* w = &grad->W1[(t - NH) * NIN];
+      atomicAdd(&grad->b1[t - NH], v[ONES_COL - 80]);
+      tmem_ld16(lane_base + TRAIN_DW + 64, u);
+      add16(w, u);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        tmem_ld16(lane_base + 128 + 64 + 16 * c, v);
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const int in = 16 * c + k;
-          if (in < NIN) atomicAdd(&grad->W1[(t - NH) * NIN + in], v[k]);
-          if (in == NIN) atomicAdd(&grad->b1[t - NH], v[k]);
-        }
-      }
+      for (int k = 0; k < 8; k += 4)
+        atomicAdd(reinterpret_cast<float4*>(w + 16 + k), make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]));
     }
-    atomicAdd(&grad->W3[t], gw3);
-    if (t < NOUT) atomicAdd(&grad->b3[t], gb3);
   }
   float l = loss_local;
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) l += __shfl_xor_sync(0xffffffffu, l, s);
-  if (lane == 0) atomicAdd(loss, l);
+  for (int s = 16; s > 0; s >>= 1) {
+    l += __shfl_xor_sync(0xffffffffu, l, s);
+    gb3[0] += __shfl_xor_sync(0xffffffffu, gb3[0], s);
+    gb3[1] += __shfl_xor_sync(0xffffffffu, gb3[1], s);
+  }
+  if (lane == 0) {
+    atomicAdd(loss, l);
+    if (!waits.aborted()) {
+      atomicAdd(&grad->b3[0], gb3[0]);
+      atomicAdd(&grad->b3[1], gb3[1]);
+    }
+  }
   if (waits.aborted() && t == 0) atomicExch(&status->error, 1);
   fence_before();
   __syncthreads();
@@ -323,6 +378,18 @@ __global__ void __launch_bounds__(TILE, 2) k_mlp_train(const __nv_bfloat16* __re
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TRAIN_TMEM_COLS)
                  : "memory");
+}
+
+// parameter i's BF16 copy
+__device__ __forceinline__ void refresh_bf16(ParamsBF16* wbf, int i, float x) {
+  const __nv_bfloat16 b = __float2bfloat16_rn(x);
+  constexpr int oW2 = offsetof(Params, W2) / 4, ob2 = offsetof(Params, b2) / 4, oW3 = offsetof(Params, W3) / 4;
+  if (i < NH * NIN)
+    wbf->W1[i / NIN * KIN + i % NIN] = b;
+  else if (i >= oW2 && i < ob2)
+    wbf->W2[i - oW2] = b;
+  else if (i >= oW3 && i < oW3 + NOUT * NH)
+    wbf->W3[i - oW3] = b;
 }
 
 // Adam on the FP32 master parameters; refreshes the BF16 copies.
@@ -340,17 +407,23 @@ __global__ void k_adam(Params* p, const Params* g, Params* m, Params* v, ParamsB
   Mm[i] = mi;
   Vv[i] = vi;
   P[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  refresh_bf16(wbf, i, P[i]);
 }
 
 __global__ void k_refresh_bf16(const Params* p, ParamsBF16* wbf) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < NH * KIN) {
-    const int r = i / KIN, c = i % KIN;
-    wbf->W1[i] = __float2bfloat16_rn(c < NIN ? p->W1[r * NIN + c] : 0.0f);
-  }
-  if (i < NH * NH) wbf->W2[i] = __float2bfloat16_rn(p->W2[i]);
-  if (i < NOUT * NH) wbf->W3[i] = __float2bfloat16_rn(p->W3[i]);
+  if (i < NPARAM) refresh_bf16(wbf, i, reinterpret_cast<const float*>(p)[i]);
 }
+
+// A training step's sums, in one allocation: cleared and read back in one operation each.
+struct LossStatus {
+  float loss;  // squared errors
+  Status status;
+};
+struct Sums {
+  Params g;  // gradients
+  LossStatus end;
+};
 
 }  // namespace closure
 }  // namespace trisk
@@ -364,10 +437,11 @@ struct TriskClosure {
   int device = 0;
   cudaStream_t stream = cudaStreamLegacy;
   Params* p = nullptr;
-  Params *g = nullptr, *m = nullptr, *v = nullptr;
+  Sums* sums = nullptr;
+  Params *g = nullptr, *m = nullptr, *v = nullptr;  // g: sums->g
   ParamsBF16* wbf = nullptr;
-  float* loss = nullptr;
-  Status* status = nullptr;
+  float* loss = nullptr;     // &sums->end.loss
+  Status* status = nullptr;  // &sums->end.status
   int64_t adam_step = 0;
   int64_t launches = 0;
   int sms = 0;              // the device's SM count (persistent grids)
@@ -378,7 +452,7 @@ struct TriskClosure {
     cudaGetDevice(&prev);
     cudaSetDevice(device);
     cudaStreamSynchronize(stream);
-    for (void* q : {(void*)p, (void*)g, (void*)m, (void*)v, (void*)wbf, (void*)loss, (void*)status})
+    for (void* q : {(void*)p, (void*)sums, (void*)m, (void*)v, (void*)wbf})
       if (q) cudaFree(q);
     if (prev >= 0) cudaSetDevice(prev);
   }
@@ -391,14 +465,16 @@ TriskClosure* checked_c(TriskClosure* c) {
   return c;
 }
 
-void check_status(TriskClosure& c) {
-  Status s{};
-  CUDA_CHECK(cudaMemcpyAsync(&s, c.status, sizeof(s), cudaMemcpyDeviceToHost, c.stream));
+// Waits for the closure's work; the loss of the last gradients call; throws if a wait gave up.
+float check_status(TriskClosure& c) {
+  LossStatus r{};
+  CUDA_CHECK(cudaMemcpyAsync(&r, &c.sums->end, sizeof(r), cudaMemcpyDeviceToHost, c.stream));
   CUDA_CHECK(cudaStreamSynchronize(c.stream));
-  if (s.error) {
+  if (r.status.error) {
     CUDA_CHECK(cudaMemset(c.status, 0, sizeof(Status)));
     throw Error(TRISK_ERR_TIMEOUT, "a bounded tensor-core wait in the closure MLP gave up");
   }
+  return r.loss;
 }
 
 // persistent grids: every resident CTA of the device, or one per tile when there are fewer
@@ -483,18 +559,20 @@ int trisk_closure_create(int32_t device, const float* params, TriskClosure** out
   c->device = device;
   DeviceGuard guard(device);
   CUDA_CHECK(cudaMalloc(&c->p, sizeof(Params)));
-  CUDA_CHECK(cudaMalloc(&c->g, sizeof(Params)));
+  CUDA_CHECK(cudaMalloc(&c->sums, sizeof(Sums)));
+  c->g = &c->sums->g;
+  c->loss = &c->sums->end.loss;
+  c->status = &c->sums->end.status;
   CUDA_CHECK(cudaMalloc(&c->m, sizeof(Params)));
   CUDA_CHECK(cudaMalloc(&c->v, sizeof(Params)));
   CUDA_CHECK(cudaMalloc(&c->wbf, sizeof(ParamsBF16)));
-  CUDA_CHECK(cudaMalloc(&c->loss, sizeof(float)));
-  CUDA_CHECK(cudaMalloc(&c->status, sizeof(Status)));
   CUDA_CHECK(cudaMemset(c->m, 0, sizeof(Params)));
   CUDA_CHECK(cudaMemset(c->v, 0, sizeof(Params)));
-  CUDA_CHECK(cudaMemset(c->status, 0, sizeof(Status)));
+  CUDA_CHECK(cudaMemset(c->sums, 0, sizeof(Sums)));
+  CUDA_CHECK(cudaMemset(c->wbf, 0, sizeof(ParamsBF16)));  // W1's padding
   if (params) CUDA_CHECK(cudaMemcpy(c->p, params, sizeof(Params), cudaMemcpyHostToDevice));
   else CUDA_CHECK(cudaMemset(c->p, 0, sizeof(Params)));
-  k_refresh_bf16<<<(NH * NH + 255) / 256, 256, 0, c->stream>>>(c->p, c->wbf);
+  k_refresh_bf16<<<(NPARAM + 255) / 256, 256, 0, c->stream>>>(c->p, c->wbf);
   CUDA_CHECK(cudaGetLastError());
   CUDA_CHECK(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   CUDA_CHECK(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -528,7 +606,7 @@ int trisk_closure_set_params(TriskClosure* closure, const float* params) {
   if (!params) throw Error(TRISK_ERR_ARGUMENT, "NULL argument");
   DeviceGuard guard(c.device);
   CUDA_CHECK(cudaMemcpyAsync(c.p, params, sizeof(Params), cudaMemcpyHostToDevice, c.stream));
-  k_refresh_bf16<<<(NH * NH + 255) / 256, 256, 0, c.stream>>>(c.p, c.wbf);
+  k_refresh_bf16<<<(NPARAM + 255) / 256, 256, 0, c.stream>>>(c.p, c.wbf);
   CUDA_CHECK(cudaGetLastError());
   CUDA_CHECK(cudaStreamSynchronize(c.stream));
   TRISK_API_END
@@ -553,13 +631,10 @@ int trisk_closure_gradients(TriskClosure* closure, const void* X, const float* t
   TriskClosure& c = *checked_c(closure);
   if (!X || !target || n <= 0) throw Error(TRISK_ERR_ARGUMENT, "bad argument");
   DeviceGuard guard(c.device);
-  CUDA_CHECK(cudaMemsetAsync(c.g, 0, sizeof(Params), c.stream));
-  CUDA_CHECK(cudaMemsetAsync(c.loss, 0, sizeof(float), c.stream));
+  CUDA_CHECK(cudaMemsetAsync(c.sums, 0, offsetof(Sums, end) + offsetof(LossStatus, status), c.stream));  // the status stays until it is read
   launch_train(c, static_cast<const __nv_bfloat16*>(X), n, target, 1.0f / (float)n);
   if (grads) CUDA_CHECK(cudaMemcpyAsync(grads, c.g, sizeof(Params), cudaMemcpyDeviceToHost, c.stream));
-  float l = 0;
-  CUDA_CHECK(cudaMemcpyAsync(&l, c.loss, sizeof(float), cudaMemcpyDeviceToHost, c.stream));
-  check_status(c);
+  const float l = check_status(c);
   if (loss) *loss = l / (float)n;
   TRISK_API_END
 }
@@ -572,9 +647,8 @@ int trisk_closure_adam(TriskClosure* closure, float lr, float beta1, float beta2
   c.adam_step++;
   const float c1 = 1.0f - powf(beta1, (float)c.adam_step), c2 = 1.0f - powf(beta2, (float)c.adam_step);
   k_adam<<<(NPARAM + 255) / 256, 256, 0, c.stream>>>(c.p, c.g, c.m, c.v, c.wbf, lr, beta1, beta2, eps, c1, c2);
-  k_refresh_bf16<<<(NH * NH + 255) / 256, 256, 0, c.stream>>>(c.p, c.wbf);
   CUDA_CHECK(cudaGetLastError());
-  c.launches += 2;
+  c.launches++;
   TRISK_API_END
 }
 

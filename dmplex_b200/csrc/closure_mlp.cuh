@@ -25,8 +25,6 @@ constexpr int HX_BYTES = 12 * HX_CHUNK;  // 96 columns: H1 (0..63) | X (64..95)
 constexpr int DD_BYTES = 16 * HX_CHUNK;  // 128 columns: dH2 (0..63) | dH1 (64..127)
 constexpr int W1_BYTES = 4 * W_CHUNK;    // 64 x 32
 constexpr int W2_BYTES = 8 * W_CHUNK;    // 64 x 64
-// + 64 B (mbarrier, TMEM address) + H2 (128 x 64 BF16) and dY (128 x 2 FP32) for training
-constexpr int SMEM_BYTES = HX_BYTES + DD_BYTES + W1_BYTES + W2_BYTES + 64 + TILE * NH * 2 + TILE * NOUT * 4;
 constexpr uint32_t TRAIN_TMEM_COLS = 256;  // two CTAs per SM share its 512 columns
 // Inference: a chunk of ones, XH (X, then H1, then H2: 8 chunks), W1, W2, b2, W3 and the barrier, 64
 // TMEM columns; six CTAs fit an SM's shared memory, and eight x 64 columns fit its TMEM, so no CTA
@@ -38,6 +36,11 @@ constexpr int W3_BYTES = 8 * W3_CHUNK;
 constexpr int FWD_SMEM_BYTES = HX_CHUNK + XH_BYTES + W1_BYTES + W2_BYTES + B2_BYTES + W3_BYTES + 64;
 constexpr uint32_t FWD_TMEM_COLS = 64;
 static_assert(FWD_SMEM_BYTES * 6 <= 220 * 1024, "six inference CTAs per SM");
+// Training: HX, H2 (8 chunks), DD, dY (2 chunks), W1, W2, b2, W3 in both orders and the barrier.
+constexpr int H2_BYTES = 8 * HX_CHUNK, DY_BYTES = 2 * HX_CHUNK;
+constexpr int SMEM_BYTES =
+    HX_BYTES + H2_BYTES + DD_BYTES + DY_BYTES + W1_BYTES + W2_BYTES + B2_BYTES + W3_BYTES + 2 * W_CHUNK + 64;
+static_assert(SMEM_BYTES * 2 <= 220 * 1024, "two training CTAs per SM");
 // A bounded tensor-core wait gives up after this long (the operations take microseconds).
 constexpr long long MBAR_WAIT_NS = 500000000LL;
 
@@ -142,6 +145,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
 #pragma unroll
   for (int k = 0; k < 32; ++k) v[k] = __uint_as_float(r[k]);
 }
+// 32 consecutive columns of this thread's lane written (complete on return)
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+      "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
+      "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]), "f"(v[16]), "f"(v[17]), "f"(v[18]),
+      "f"(v[19]), "f"(v[20]), "f"(v[21]), "f"(v[22]), "f"(v[23]), "f"(v[24]), "f"(v[25]), "f"(v[26]), "f"(v[27]),
+      "f"(v[28]), "f"(v[29]), "f"(v[30]), "f"(v[31])
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 // two
 __device__ __forceinline__ void tmem_ld2(uint32_t taddr, float& a, float& b) {
   uint32_t r[2];
@@ -159,18 +174,6 @@ __device__ __forceinline__ float tanh_approx(float x) {
 // gelu(x) = x/2 (1 + tanh(u)), u = sqrt(2/pi) (x + 0.044715 x^3) (Hendrycks and Gimpel 2016)
 constexpr float GELU_C0 = 0.7978845608028654f;   // sqrt(2/pi)
 constexpr float GELU_C1 = 0.035677408136300125f;  // 0.044715 sqrt(2/pi)
-__device__ __forceinline__ float gelu(float x) {
-  const float u = x * fmaf(GELU_C1, x * x, GELU_C0);
-  const float h = 0.5f * x;
-  return fmaf(h, tanh_approx(u), h);
-}
-// d gelu / dx = (1 + t)/2 + x/2 (1 - t^2) du/dx,  du/dx = sqrt(2/pi) (1 + 3 * 0.044715 x^2)
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float x2 = x * x;
-  const float t = tanh_approx(x * fmaf(GELU_C1, x2, GELU_C0));
-  const float du = fmaf(3.0f * GELU_C1, x2, GELU_C0);
-  return fmaf(0.5f * x * fmaf(-t, t, 1.0f), du, fmaf(0.5f, t, 0.5f));
-}
 // Two FP32 values at once (Blackwell's packed instructions, each half rounded as the scalar one):
 // half the issue slots, which the epilogues of the network run out of.
 struct F2 {
@@ -204,12 +207,22 @@ __device__ __forceinline__ F2 tanh2(F2 x) {
   unpack2(x, a, b);
   return pack2(tanh_approx(a), tanh_approx(b));
 }
-// gelu(2h) of both halves, bit for bit gelu(): x = 2h, so x/2 is h itself, and u = x (C0 + C1 x^2)
-// = h (2 C0 + 8 C1 h^2), scaled by powers of two throughout. The caller halves the weights and
-// biases that form x (exact in binary), which saves the multiplication by 1/2.
+// gelu(2h) of both halves: x/2 is h itself, and u = x (C0 + C1 x^2) = h (2 C0 + 8 C1 h^2), scaled by
+// powers of two throughout. The caller halves the weights and biases that form x (exact in
+// binary), which saves the multiplication by 1/2.
 __device__ __forceinline__ F2 gelu2_of_half(F2 h) {
   const F2 u = mul2(h, fma2(pack2(8.0f * GELU_C1, 8.0f * GELU_C1), mul2(h, h), pack2(2.0f * GELU_C0, 2.0f * GELU_C0)));
   return fma2(h, tanh2(u), h);
+}
+// gelu(2h) and its derivative at 2h, of both halves: with x = 2h and t = tanh(u),
+// d gelu / dx = (1 + t)/2 + h (1 - t^2) du/dx, du/dx = C0 + 3 C1 x^2 = C0 + 12 C1 h^2
+__device__ __forceinline__ F2 gelu2_of_half(F2 h, F2& grad) {
+  const F2 s = mul2(h, h);
+  const F2 t = tanh2(mul2(h, fma2(pack2(8.0f * GELU_C1, 8.0f * GELU_C1), s, pack2(2.0f * GELU_C0, 2.0f * GELU_C0))));
+  const F2 one_t2 = fma2(F2{t.v ^ 0x8000000080000000ull}, t, pack2(1.0f, 1.0f));
+  const F2 du = fma2(pack2(12.0f * GELU_C1, 12.0f * GELU_C1), s, pack2(GELU_C0, GELU_C0));
+  grad = fma2(mul2(h, one_t2), du, fma2(pack2(0.5f, 0.5f), t, pack2(0.5f, 0.5f)));
+  return fma2(h, t, h);
 }
 // the two halves rounded to BF16 (low half first)
 __device__ __forceinline__ uint32_t bf16x2(F2 x) {
@@ -218,50 +231,13 @@ __device__ __forceinline__ uint32_t bf16x2(F2 x) {
   const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&p);
 }
-__device__ __forceinline__ float bf(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-
 __device__ __forceinline__ uint32_t tile_off(int r, int c, int chunk) {
   return (uint32_t)((c >> 3) * chunk + (r >> 3) * 128 + (r & 7) * 16 + (c & 7) * 2);
-}
-
-// 8 consecutive columns (c0 multiple of 8) of row r as one 16-byte store
-__device__ __forceinline__ void store8(unsigned char* base, int r, int c0, int chunk, const float* v) {
-  uint4 q;
-  __nv_bfloat162 p0 = __floats2bfloat162_rn(v[0], v[1]), p1 = __floats2bfloat162_rn(v[2], v[3]),
-                 p2 = __floats2bfloat162_rn(v[4], v[5]), p3 = __floats2bfloat162_rn(v[6], v[7]);
-  q.x = *reinterpret_cast<uint32_t*>(&p0);
-  q.y = *reinterpret_cast<uint32_t*>(&p1);
-  q.z = *reinterpret_cast<uint32_t*>(&p2);
-  q.w = *reinterpret_cast<uint32_t*>(&p3);
-  *reinterpret_cast<uint4*>(base + tile_off(r, c0, chunk)) = q;
 }
 
 struct Status {
   int error;  // 1: a bounded tensor-core wait gave up
 };
-
-// W1 (64 x 32, inputs padded with 0) and W2 (64 x 64) as K-major B operands; biases and W3 (unit
-// by unit, the two outputs' weights side by side)
-__device__ __forceinline__ void load_weights(unsigned char* W1s, unsigned char* W2s, float* sb1, float* sb2,
-                                             float* sw3, float* sb3, const ParamsBF16* __restrict__ wbf,
-                                             const Params* __restrict__ p, int t) {
-  for (int idx = t; idx < NH * 4; idx += TILE) {
-    const int r = idx >> 2, c0 = (idx & 3) * 8;
-    *reinterpret_cast<uint4*>(W1s + tile_off(r, c0, W_CHUNK)) =
-        *reinterpret_cast<const uint4*>(wbf->W1 + r * KIN + c0);
-  }
-  for (int idx = t; idx < NH * 8; idx += TILE) {
-    const int r = idx >> 3, c0 = (idx & 7) * 8;
-    *reinterpret_cast<uint4*>(W2s + tile_off(r, c0, W_CHUNK)) =
-        *reinterpret_cast<const uint4*>(wbf->W2 + r * NH + c0);
-  }
-  for (int idx = t; idx < NH; idx += TILE) {
-    sb1[idx] = p->b1[idx];
-    sb2[idx] = p->b2[idx];
-  }
-  for (int idx = t; idx < NOUT * NH; idx += TILE) sw3[NOUT * (idx % NH) + idx / NH] = __bfloat162float(wbf->W3[idx]);
-  if (t < NOUT) sb3[t] = p->b3[t];
-}
 
 // 8 BF16 values halved (exact in binary)
 __device__ __forceinline__ uint4 half_bf16x8(const __nv_bfloat16* p) {
@@ -284,6 +260,32 @@ __device__ __forceinline__ uint4 split_bf16(float x) {
 }
 // columns 0..2 of a chunk row = 1: what split_bf16's three terms are multiplied with
 __device__ __forceinline__ uint4 three_ones() { return make_uint4(0x3F803F80u, 0x3F80u, 0u, 0u); }
+
+// The network's weights as K-major B operands: W1 with b1 in its padding, W2 and b2, all halved as
+// gelu2_of_half takes them, and W3 (16 rows, two used).
+__device__ __forceinline__ void load_weights(unsigned char* W1s, unsigned char* W2s, unsigned char* B2s,
+                                             unsigned char* W3s, const ParamsBF16* __restrict__ wbf,
+                                             const Params* __restrict__ p, int t) {
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (int idx = t; idx < NH * 4; idx += TILE) {
+    const int r = idx >> 2, c = idx & 3;
+    *reinterpret_cast<uint4*>(W1s + tile_off(r, 8 * c, W_CHUNK)) =
+        c < 3 ? half_bf16x8(wbf->W1 + r * KIN + 8 * c) : split_bf16(0.5f * p->b1[r]);
+  }
+  for (int idx = t; idx < NH * 8; idx += TILE) {
+    const int r = idx >> 3, c0 = (idx & 7) * 8;
+    *reinterpret_cast<uint4*>(W2s + tile_off(r, c0, W_CHUNK)) = half_bf16x8(wbf->W2 + r * NH + c0);
+  }
+  {
+    const int r = t >> 1, c = t & 1;  // 64 rows x 2 chunks
+    *reinterpret_cast<uint4*>(B2s + tile_off(r, 8 * c, W_CHUNK)) = c == 0 ? split_bf16(0.5f * p->b2[r]) : zero;
+  }
+  {
+    const int r = t >> 3, c = t & 7;  // 16 rows x 8 chunks
+    *reinterpret_cast<uint4*>(W3s + tile_off(r, 8 * c, W3_CHUNK)) =
+        r < NOUT ? *reinterpret_cast<const uint4*>(wbf->W3 + r * NH + 8 * c) : zero;
+  }
+}
 
 // The bounded tensor-core waits of a CTA. wait() records a give-up in the CTA's shared abort
 // word; every thread reads that word only right after a CTA-wide barrier, so all threads
@@ -336,8 +338,7 @@ struct InferStatic {
   int abort;
 };
 
-// Tensor memory, the mbarrier and the weights (W1, W2 and their biases halved, as gelu2_of_half
-// takes them); returns the CTA's TMEM base address.
+// Tensor memory, the mbarrier and the weights; returns the CTA's TMEM base address.
 __device__ __forceinline__ uint32_t infer_setup(const InferSmem& S, InferStatic& st, const ParamsBF16* wbf,
                                                 const Params* p) {
   const int t = threadIdx.x, warp = t >> 5;
@@ -352,26 +353,8 @@ __device__ __forceinline__ uint32_t infer_setup(const InferSmem& S, InferStatic&
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     st.abort = 0;
   }
-  const uint4 zero = make_uint4(0, 0, 0, 0);
   *reinterpret_cast<uint4*>(S.ones + tile_off(t, 0, HX_CHUNK)) = three_ones();
-  for (int idx = t; idx < NH * 4; idx += TILE) {  // W1's inputs, then b1 in the padding
-    const int r = idx >> 2, c = idx & 3;
-    *reinterpret_cast<uint4*>(S.W1s + tile_off(r, 8 * c, W_CHUNK)) =
-        c < 3 ? half_bf16x8(wbf->W1 + r * KIN + 8 * c) : split_bf16(0.5f * p->b1[r]);
-  }
-  for (int idx = t; idx < NH * 8; idx += TILE) {
-    const int r = idx >> 3, c0 = (idx & 7) * 8;
-    *reinterpret_cast<uint4*>(S.W2s + tile_off(r, c0, W_CHUNK)) = half_bf16x8(wbf->W2 + r * NH + c0);
-  }
-  {
-    const int r = t >> 1, c = t & 1;  // 64 rows x 2 chunks
-    *reinterpret_cast<uint4*>(S.B2s + tile_off(r, 8 * c, W_CHUNK)) = c == 0 ? split_bf16(0.5f * p->b2[r]) : zero;
-  }
-  {
-    const int r = t >> 3, c = t & 7;  // 16 rows x 8 chunks
-    *reinterpret_cast<uint4*>(S.W3s + tile_off(r, 8 * c, W3_CHUNK)) =
-        r < NOUT ? *reinterpret_cast<const uint4*>(wbf->W3 + r * NH + 8 * c) : zero;
-  }
+  load_weights(S.W1s, S.W2s, S.B2s, S.W3s, wbf, p, t);
   if (t < NOUT) st.b3[t] = p->b3[t];
   fence_async_smem();
   fence_before();

@@ -80,6 +80,33 @@ def test_forward_and_gradients_match_oracle(require_gpu, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [31, 129, 38017])
+def test_biases_and_ragged_rows_match_oracle(require_gpu, n):
+    """Biases of the size of the pre-activations (three BF16 terms each in the kernels, so exact) at
+    row counts that leave part of a tile and, at the largest, one more tile for some CTAs; the
+    tolerances of the test above."""
+    import torch
+    import dmplex_b200.closure as cl
+    X, T = _data(n, n + 1)
+    p = co.unpack(co.init_params(11))
+    rng = np.random.default_rng(n)
+    for name in ("b1", "b2", "b3"):
+        p[name] = rng.standard_normal(p[name].shape)
+    mlp = cl.ClosureMLP(co.pack(p).astype(np.float32))
+    Xd = torch.from_numpy(X.astype(np.float32)).to(torch.bfloat16).cuda().contiguous()
+    Td = torch.from_numpy(T.astype(np.float32)).cuda().contiguous()
+    pf = mlp.params().astype(np.float64)
+    Yo, _ = co.forward(pf, X)
+    assert _rel(mlp.forward(Xd).cpu().numpy(), Yo) <= 1e-2
+    g, loss = mlp.gradients(Xd, Td)
+    go, lo = co.gradients(pf, X, T)
+    assert abs(loss - lo) <= 1e-2 * lo
+    gb, gob = _blocks(g), _blocks(go)
+    for name, _ in co.SHAPES:
+        assert _rel(gb[name], gob[name]) <= 2e-2, name
+
+
+@pytest.mark.gpu
 def test_training_reduces_loss(require_gpu):
     import torch
     import dmplex_b200.closure as cl
