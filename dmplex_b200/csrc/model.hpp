@@ -101,6 +101,8 @@ struct TriskModel {
   double phase_bytes[3] = {0, 0, 0};
   double pv_table_bytes_saved = 0;  // k_tend bytes per launch the derived PV edges do not read
   cudaEvent_t caller_ev = nullptr;  // for order_after_caller
+  char* pinned = nullptr;           // one state of pinned host memory, for copies of pageable states
+  cudaEvent_t stage_ev[4] = {};     // its pieces' last copies
   char* table_base = nullptr;       // the packed table block (tendency phase's tables first)
   size_t table_block_bytes = 0;     // its part the kernels read
   size_t l2_keep_bytes = 0;         // prefix loaded with the L2 evict-last policy
@@ -116,8 +118,19 @@ struct TriskModel {
       cudaStreamSynchronize(stream);
       cudaStreamDestroy(stream);
     }
+    for (cudaEvent_t ev : stage_ev)
+      if (ev) cudaEventDestroy(ev);
+    if (pinned) cudaFreeHost(pinned);
     for (void* p : allocations) cudaFree(p);
     if (prev >= 0) cudaSetDevice(prev);
+  }
+
+  // the pinned buffer and its events, made on the first copy that uses them
+  char* pinned_stage() {
+    for (cudaEvent_t& ev : stage_ev)
+      if (!ev) CUDA_CHECK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    if (!pinned) CUDA_CHECK(cudaMallocHost((void**)&pinned, (size_t)N * sizeof(double)));
+    return pinned;
   }
 
   template <class T>
