@@ -527,7 +527,7 @@ int trisk_mpas_create(const TriskMpasTables* t, int32_t device, int32_t levels_p
   if (t->vertical < 0 || t->vertical > 2) throw Error(TRISK_ERR_ARGUMENT, "vertical must be 0, 1 or 2");
   if (t->five_band && t->vertical == 0)
     throw Error(TRISK_ERR_ARGUMENT, "the five-band solver needs the vector-invariant vertical advection");
-  const int lpt = levels_per_thread == 0 ? 8 : levels_per_thread;
+  int lpt = levels_per_thread == 0 ? 8 : levels_per_thread;
   if (lpt != 1 && lpt != 2 && lpt != 4 && lpt != 8 && lpt != 16)
     throw Error(TRISK_ERR_ARGUMENT, "levels_per_thread must be 0 (default), 1, 2, 4, 8 or 16");
   const int64_t cells_levels = t->nc * (t->nlev + 1), edges_levels = t->ne * (t->nlev + 1);
@@ -541,8 +541,17 @@ int trisk_mpas_create(const TriskMpasTables* t, int32_t device, int32_t levels_p
   if (device < 0 || device >= ndev) throw Error(TRISK_ERR_ARGUMENT, "no such CUDA device");
   auto m = std::make_unique<TriskMpas>();
   m->device = device;
-  m->lpt = lpt;
   DeviceGuard guard(device);
+  if (levels_per_thread == 0) {
+    // Longer runs of levels read the tables less often, shorter ones make more blocks: runs of 8, halved
+    // (to 2 at least) while the narrowest phase, the cells, has fewer than four blocks an SM.
+    // Measured with 30 levels, us a call at 8 / 4 / 2 / 1 levels: hexagon 7 1265 / 1300 / 1530 / 1869,
+    // hexagon 6 380 / 376 / 372 / 387, hexagon 5 145 / 121 / 120 / 125, hexagon 4 97 / 69 / 61 / 62.
+    int sms = 0;
+    CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    while (lpt > 2 && cdiv(t->nc, MB) * cdiv(t->nlev, lpt) < 4 * (int64_t)sms) lpt /= 2;
+  }
+  m->lpt = lpt;
   const int64_t nc = t->nc, ne = t->ne, nv = t->nv, nl = t->nlev;
   const int64_t ldc = round_up(nc, 32), lde = round_up(ne, 32), ldv = round_up(nv, 32);
   MpasTables& T = m->T;

@@ -353,7 +353,7 @@ typedef struct {
 } TriskMpasFields;
 typedef struct TriskMpas TriskMpas;
 /* Uploads the tables once. levels_per_thread: levels each thread walks with its neighbour
- * tables in registers (0 = 8; 1, 2, 4, 8 or 16). Tables wider than 10 edges per cell, 4 per
+ * tables in registers (1, 2, 4, 8 or 16; 0: 8, fewer on meshes too small to fill the device). Tables wider than 10 edges per cell, 4 per
  * vertex or 18 TRiSK neighbours return TRISK_ERR_UNSUPPORTED. */
 int trisk_mpas_create(const TriskMpasTables* tables, int32_t device, int32_t levels_per_thread, TriskMpas** out);
 void trisk_mpas_destroy(TriskMpas* ops);
