@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(TILE, 2) k_mlp_train(const __nv_bfloat16* __re
                                                        float* loss, float inv_n, Status* status) {
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* HX = smem;
-  unsigned char* H2 = HX + HX_BYTES;  // after HX's ones chunk, before DD: both are read across the border
+  unsigned char* H2 = HX + HX_BYTES;  // directly before DD: dW3's operand reaches into it (unused rows)
   unsigned char* DD = H2 + H2_BYTES;
   unsigned char* DY = DD + DD_BYTES;
   unsigned char* W1s = DY + DY_BYTES;
@@ -152,8 +152,6 @@ __global__ void __launch_bounds__(TILE, 2) k_mlp_train(const __nv_bfloat16* __re
     *reinterpret_cast<uint4*>(W3t + tile_off(t, 0, W_CHUNK)) = make_uint4(a | (a << 16), a | (b << 16), b | (b << 16), 0);
     *reinterpret_cast<uint4*>(W3t + tile_off(t, 8, W_CHUNK)) = make_uint4(0, 0, 0, 0);
   }
-  // H2's first chunk is b2's second K chunk (against zeros) before a tile has filled it
-  *reinterpret_cast<uint4*>(H2 + tile_off(t, 0, HX_CHUNK)) = make_uint4(0, 0, 0, 0);
   *reinterpret_cast<uint4*>(DY + tile_off(t, 8, HX_CHUNK)) = make_uint4(0, 0, 0, 0);
   if (t < NOUT) sb3[t] = p->b3[t];
   fence_async_smem();
@@ -230,7 +228,8 @@ __global__ void __launch_bounds__(TILE, 2) k_mlp_train(const __nv_bfloat16* __re
       for (int kk = 0; kk < 4; ++kk)
         mma_bf16(tmem + 64, sdesc(hx + 2 * kk * HX_CHUNK, HX_CHUNK, 128), sdesc(w2 + 2 * kk * W_CHUNK, W_CHUNK, 128), ID,
                  kk);
-      mma_bf16(tmem + 64, sdesc(hx + 11 * HX_CHUNK, HX_CHUNK, 128), sdesc(b2, W_CHUNK, 128), ID, 1);
+      // the ones, and W1's first chunk against zeros
+      mma_bf16(tmem + 64, sdesc(hx + 11 * HX_CHUNK, w1 - (hx + 11 * HX_CHUNK), 128), sdesc(b2, W_CHUNK, 128), ID, 1);
       mma_commit(waits.mb);
     }
     waits.wait(true);

@@ -320,7 +320,7 @@ struct MmaWaits {
 // 65 % busy and the tanh unit at 64 %. So a bias is three BF16 terms (exact) against columns of
 // ones (b1 in X's padding, b2 in one more K step), and the output layer is a third MMA on H2.
 struct InferSmem {
-  unsigned char* ones;  // directly before XH: the second chunk of its K step is H1's first, against zeros
+  unsigned char* ones;  // the second chunk of its K step is W1's first, against zeros
   unsigned char* XH;
   unsigned char* W1s;
   unsigned char* W2s;
@@ -424,7 +424,7 @@ __device__ __forceinline__ bool infer_tile(const InferSmem& S, const InferStatic
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
       mma_bf16(tmem, sdesc(xh + 2 * kk * HX_CHUNK, HX_CHUNK, 128), sdesc(w2 + 2 * kk * W_CHUNK, W_CHUNK, 128), ID, kk);
-    mma_bf16(tmem, sdesc(smem_u32(S.ones), HX_CHUNK, 128), sdesc(smem_u32(S.B2s), W_CHUNK, 128), ID, 1);
+    mma_bf16(tmem, sdesc(smem_u32(S.ones), w1 - smem_u32(S.ones), 128), sdesc(smem_u32(S.B2s), W_CHUNK, 128), ID, 1);
     mma_commit(waits.mb);
   }
   waits.wait(true);
