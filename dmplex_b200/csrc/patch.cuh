@@ -114,8 +114,9 @@ __device__ __forceinline__ void publish(Tagged* p, double x, unsigned version) {
   asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"((b & 0xFFFFFFFFull) | t), "l"((b >> 32) | t)
                : "memory");
 }
-// The value of `version` at p, waited for; false if the wait gave up: after a second (or 2^31
-// polls, which the clock always beats), or when another block's has.
+// The value of `version` at p, waited for; false if the wait gave up: after ten seconds (or 2^31
+// polls, which the clock always beats; a neighbour may have to wait for an SM that another
+// stream's kernel holds), or when another block's has.
 __device__ __forceinline__ bool receive(const Tagged* p, unsigned version, double& x, int* err) {
   long long start = 0;
   for (unsigned i = 1;; ++i) {
@@ -128,7 +129,7 @@ __device__ __forceinline__ bool receive(const Tagged* p, unsigned version, doubl
     if ((i & 255u) == 0) {
       const long long now = barrier_ns();
       if (start == 0) start = now;
-      if (now - start > 1000000000LL || *reinterpret_cast<volatile int*>(err) != 0 || i >= (1u << 31)) {
+      if (now - start > 10000000000LL || *reinterpret_cast<volatile int*>(err) != 0 || i >= (1u << 31)) {
         atomicExch(err, 1);
         x = 0.0;
         return false;
