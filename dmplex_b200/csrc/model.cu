@@ -253,9 +253,11 @@ void ensure_graph(TriskModel& m, double dt) {
 }
 
 constexpr int PERSISTENT_BLOCK = 256;
-// The smallest mesh whose RK4 runs take the patches: below it (hexagon 3: 642 cells) a patch has
-// four cells and a halo of twenty, and the twelve launches a step stay.
-constexpr int64_t PATCH_RK4_MIN_CELLS = 1024;
+// Below this many cells (hexagon 3 has 642) runs of fewer steps than PATCH_RUN_STEPS stay with the
+// twelve launches a step that a caller of one step at a time counts; longer runs, and all runs of
+// larger meshes, take the patches. Measured, us a step in runs of 200, launches / patches: hexagon 2
+// 16.5 / 7.6, hexagon 3 18.0 / 8.3, hexagon 4 18.6 / 7.9, hexagon 5 21.9 / 10.5.
+constexpr int64_t PATCH_RK4_MIN_CELLS = 1024, PATCH_RUN_STEPS = 8;
 
 // All nsteps RK4 steps as one cooperative launch of k_rk4_persistent.
 void run_persistent(TriskModel& m, double dt, int64_t nsteps) {
@@ -283,7 +285,7 @@ void run_persistent(TriskModel& m, double dt, int64_t nsteps) {
 void run_steps(TriskModel& m, double dt, int64_t nsteps) {
   if (m.persistent) {
     run_persistent(m, dt, nsteps);
-  } else if (m.use_patches) {
+  } else if (m.use_patches && (m.nc >= PATCH_RK4_MIN_CELLS || nsteps >= PATCH_RUN_STEPS)) {
     patch_rk4(m, dt, nsteps);
   } else if (m.use_graph) {
     ensure_graph(m, dt);
@@ -848,7 +850,7 @@ void finish_create(TriskModel& m, const Coefficients& C, const std::vector<V3>* 
   CUDA_CHECK(cudaMemcpy(m.vertex_o2n, m.vert_o2n.data(), m.nv * sizeof(int32_t), cudaMemcpyHostToDevice));
   m.C = C;
   choose_patches(m);
-  m.use_patches = m.patches.runs && m.use_graph && !(cfg && cfg->block) && m.nc >= PATCH_RK4_MIN_CELLS;
+  m.use_patches = m.patches.runs && m.use_graph && !(cfg && cfg->block);
   CUDA_CHECK(cudaDeviceSynchronize());
 }
 

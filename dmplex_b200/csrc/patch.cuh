@@ -11,7 +11,7 @@
 //
 // Measured (CUDA events around a synchronous call of 200 steps, us per RK4 step, before / after):
 // hexagon 4 18.6 / 8.3 (TRiSK, cell K), 20.7 / 8.3 (Gassmann, vertex K); hexagon 5 21.5 / 10.4 and
-// 22.4 / 11.0. Of a stage's 5 us on hexagon 5 the exchange of the halo takes about 1.5, the three
+// 22.4 / 11.0. Of a stage's 2.6 us on hexagon 5 the exchange of the halo takes about 1.5, the three
 // phases 0.4 each: latency of barriers, shared-memory gathers and the FP64 sums. Larger meshes stay
 // with the launches: the tables no longer fit, and with them read from L2 or streamed from HBM in
 // every stage the patches measured 37 to 53 us on hexagon 6 (launches: 37 to 45) and 118 to 208 on

@@ -335,8 +335,8 @@ def test_config_level7_gassmann_vertex(require_gpu):
                                              (2, "trisk", "vertex", False), (3, "gassmann_mean", "vertex", False),
                                              (4, "trisk", "mixed", False), (5, "gassmann", "mixed", True)])
 def test_patches_bitwise(require_gpu, n, pv, ke, reorder):
-    """The patches (whole tendencies, and from hexagon 4 whole RK4 runs, from shared memory)
-    against the oracle and the three-launch tendency, bit for bit: the smallest meshes (patches
+    """The patches (whole tendencies, and RK4 runs from hexagon 4 or of eight steps, from shared
+    memory) against the oracle and the three-launch tendency, bit for bit: the smallest meshes (patches
     of four cells, a single block), numberings that are not compact, and a run of one launch."""
     import torch
     from oracle.oracle import Oracle
@@ -364,3 +364,8 @@ def test_patches_bitwise(require_gpu, n, pv, ke, reorder):
     o.rk4_step(ref, dt, 5)
     o.rk4_step(ref, dt / 2, 1)
     assert np.array_equal(a, ref) and np.array_equal(b, ref)
+    before = m.launch_count()
+    d.rk4_step(a, dt, d.tendency, d.RK4Cache(a), m, nsteps=8)  # one launch on every mesh
+    assert m.launch_count() - before <= 3
+    o.rk4_step(ref, dt, 8)
+    assert np.array_equal(a, ref)
