@@ -9,7 +9,7 @@
 // gathers from there with 16-bit local indices. Every value is formed by the expressions of
 // kernels.cuh in the same order, so results are the same bit for bit.
 //
-// Measured (CUDA events around a synchronous call of 200 steps, us per RK4 step, before / after):
+// Measured (wall clock around a synchronous call of 200 steps, us per RK4 step, before / after):
 // hexagon 4 18.6 / 8.3 (TRiSK, cell K), 20.7 / 8.3 (Gassmann, vertex K); hexagon 5 21.5 / 10.4 and
 // 22.4 / 11.0. Of a stage's 2.6 us on hexagon 5 the exchange of the halo takes about 1.5, the three
 // phases 0.4 each: latency of barriers, shared-memory gathers and the FP64 sums. Larger meshes stay
@@ -138,39 +138,6 @@ __device__ __forceinline__ bool receive(const Tagged* p, unsigned version, doubl
   }
 }
 
-template <class R, int P>
-__device__ __forceinline__ void ldcg_members(const R* p, double (&x)[P]) {
-  if constexpr (P == 1) {
-    x[0] = (double)__ldcg(p);
-  } else if constexpr (sizeof(R) == 8) {
-#pragma unroll
-    for (int q = 0; q < P; q += 2) {
-      const double2 v = __ldcg(reinterpret_cast<const double2*>(p + q));
-      x[q] = v.x;
-      x[q + 1] = v.y;
-    }
-  } else if constexpr (P == 2) {
-    const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
-    x[0] = v.x;
-    x[1] = v.y;
-  } else {
-    const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
-    x[0] = v.x;
-    x[1] = v.y;
-    x[2] = v.z;
-    x[3] = v.w;
-  }
-}
-
-// the value a storage of type R would hold
-template <class R, int P>
-__device__ __forceinline__ void round_to(double (&x)[P]) {
-  if constexpr (sizeof(R) == 4) {
-#pragma unroll
-    for (int p = 0; p < P; ++p) x[p] = (double)(float)x[p];
-  }
-}
-
 __device__ __forceinline__ void prefetch_l2(const char* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
@@ -190,233 +157,145 @@ struct PatchRow {
 constexpr int PATCH_PUBLISH = 0x8000;  // in a packed index: the owned entity is in some halo
 constexpr int PATCH_INDEX = 0x7FFF;
 
-// A patch's vectors in shared memory, [entity][MC] doubles: the stage state u, h; F, q of the
-// edges and B of the cells; the vertex values (TRiSK q_v, h_v, K_v; Gassmann zeta_v, h_v, K_v).
-// Without APART, F takes the place of u (an edge's F is formed from its own u; the cells, which
-// read other edges' u, come first) and, with no cell part in K, B that of h.
-template <int PV, int KE, int MC, bool APART>
+// A patch's vectors in shared memory: the stage state u, h; F, q of the edges and B of the cells; the
+// vertex values (TRiSK q_v, h_v, K_v; Gassmann zeta_v, h_v, K_v). Without APART, F takes the place of
+// u (an edge's F is formed from its own u; the cells, which read other edges' u, come first) except
+// with the cell K alone, and, with no cell part in K, B that of h.
+template <int PV, int KE, bool APART>
 struct PatchVectors {
   using W = PatchRows<PV, KE>;
   static constexpr bool F_OWN = APART || KE == KE_CELL, B_OWN = APART || W::CELL;
   double *u, *h, *q, *v0, *v1, *v2, *F, *B;
   __device__ __forceinline__ PatchVectors(double* sm, const PatchDesc& D) {
     u = sm;
-    h = u + (size_t)D.nSE * MC;
-    q = h + (size_t)D.nSC * MC;
-    v0 = q + (size_t)D.nLE * MC;
-    v1 = v0 + (size_t)D.nLV * MC;
-    v2 = v1 + (size_t)D.nLV * MC;
-    double* p = v0 + (size_t)W::VARRAYS * D.nLV * MC;
+    h = u + D.nSE;
+    q = h + D.nSC;
+    v0 = q + D.nLE;
+    v1 = v0 + D.nLV;
+    v2 = v1 + D.nLV;
+    double* p = v0 + W::VARRAYS * D.nLV;
     F = F_OWN ? p : u;
-    B = B_OWN ? p + (F_OWN ? (size_t)D.nLE * MC : 0) : h;
+    B = B_OWN ? p + (F_OWN ? D.nLE : 0) : h;
   }
 };
 
-// Thread t of a phase over [entity][MC]: the entity and its first member, P members a thread.
-template <int MC, int P>
-__device__ __forceinline__ void patch_slot(int t, int& i, int& mm) {
-  constexpr int L = MC / P;
-  if constexpr (L == 1) {
-    i = t;
-    mm = 0;
-  } else {
-    i = t / L;
-    mm = (t % L) * P;
-  }
-}
-
 // vertices: zeta_v, h_v, q_v, K_v
-template <int PV, int KE, class R, int MC, int P, class Vec>
+template <int PV, int KE, class Vec>
 __device__ __forceinline__ void patch_vertex(const PatchRow<PatchRows<PV, KE>::VI, PatchRows<PV, KE>::VD>& r,
-                                             const Vec& S, int v, int mm) {
+                                             const Vec& S, int v) {
   using W = PatchRows<PV, KE>;
-  double uu[VW][P], hh[VW][P], z[P], eta[P], q[P], kv[P];
+  double u[VW], z = 0.0, eta = 0.0;
 #pragma unroll
-  for (int k = 0; k < VW; ++k) {
-    ld_members<double, P>(S.u + r.ix[k] * MC + mm, uu[k]);
-    ld_members<double, P>(S.h + r.ix[VW + k] * MC + mm, hh[k]);
-  }
+  for (int k = 0; k < VW; ++k) u[k] = S.u[r.ix[k]];
 #pragma unroll
-  for (int p = 0; p < P; ++p) {
-    z[p] = 0.0;
-    eta[p] = 0.0;
+  for (int k = 0; k < VW; ++k) z += r.w[k] * u[k];
 #pragma unroll
-    for (int k = 0; k < VW; ++k) z[p] += r.w[k] * uu[k][p];
-#pragma unroll
-    for (int k = 0; k < VW; ++k) eta[p] += r.w[VW + k] * hh[k][p];
-    if (W::TR) q[p] = (z[p] + r.w[W::VD - 1]) / eta[p];
-    if (W::VERT) {
-      kv[p] = 0.0;
-#pragma unroll
-      for (int k = 0; k < VW; ++k) kv[p] += r.w[(W::VERT ? 6 : 0) + k] * (uu[k][p] * uu[k][p]);
-    }
-  }
-  const int o = v * MC + mm;
-  if (W::TR) {
-    round_to<R, P>(q);
-    st_members<double, P>(S.v0 + o, q);
-  } else {
-    round_to<R, P>(z);
-    st_members<double, P>(S.v0 + o, z);
-  }
-  if (!W::TR || W::VERT) {
-    round_to<R, P>(eta);
-    st_members<double, P>(S.v1 + o, eta);
-  }
+  for (int k = 0; k < VW; ++k) eta += r.w[VW + k] * S.h[r.ix[VW + k]];
+  S.v0[v] = W::TR ? (z + r.w[W::VD - 1]) / eta : z;
+  if (!W::TR || W::VERT) S.v1[v] = eta;
   if (W::VERT) {
-    round_to<R, P>(kv);
-    st_members<double, P>(S.v2 + o, kv);
+    double kv = 0.0;
+#pragma unroll
+    for (int k = 0; k < VW; ++k) kv += r.w[(W::VERT ? 6 : 0) + k] * (u[k] * u[k]);
+    S.v2[v] = kv;
   }
 }
 
 // edges: the mass flux F and the edge PV q
-template <int PV, int KE, class R, int MC, int P, class Vec>
+template <int PV, int KE, class Vec>
 __device__ __forceinline__ void patch_edge(const PatchRow<PatchRows<PV, KE>::FEI, PatchRows<PV, KE>::FED>& r,
-                                           const Vec& S, int e, int mm) {
+                                           const Vec& S, int e) {
   using W = PatchRows<PV, KE>;
-  constexpr int wV = W::CELL ? 2 : 0, wR = W::TR ? 0 : wV + (W::VERT ? 2 : 0);
-  double ue[P], hv0[P], hv1[P], hc0[P], hc1[P], a0[P], a1[P], Fo[P], qo[P];
-  ld_members<double, P>(S.u + e * MC + mm, ue);
-  ld_members<double, P>(S.v0 + r.ix[0] * MC + mm, a0);
-  ld_members<double, P>(S.v0 + r.ix[1] * MC + mm, a1);
+  constexpr int wV = W::CELL ? 2 : 0, wR = W::TR ? 0 : wV + (W::VERT ? 2 : 0), iC = W::CELL ? 2 : 0;
+  const double ue = S.u[e], a0 = S.v0[r.ix[0]], a1 = S.v0[r.ix[1]];
+  double hv0 = 0.0, hv1 = 0.0, hc0 = 0.0, hc1 = 0.0;
   if (W::VERT || !W::TR) {
-    ld_members<double, P>(S.v1 + r.ix[0] * MC + mm, hv0);
-    ld_members<double, P>(S.v1 + r.ix[1] * MC + mm, hv1);
+    hv0 = S.v1[r.ix[0]];
+    hv1 = S.v1[r.ix[1]];
   }
   if (W::CELL) {
-    ld_members<double, P>(S.h + r.ix[W::CELL ? 2 : 0] * MC + mm, hc0);
-    ld_members<double, P>(S.h + r.ix[W::CELL ? 3 : 0] * MC + mm, hc1);
+    hc0 = S.h[r.ix[iC]];
+    hc1 = S.h[r.ix[iC + (W::CELL ? 1 : 0)]];
   }
-#pragma unroll
-  for (int p = 0; p < P; ++p) {
-    double he;
-    if (KE == KE_CELL)
-      he = r.w[0] * hc0[p] + r.w[1] * hc1[p];
-    else if (KE == KE_VERTEX)
-      he = r.w[wV] * hv0[p] + r.w[wV + 1] * hv1[p];
-    else
-      he = r.w[0] * hc0[p] + r.w[1] * hc1[p] + r.w[wV] * hv0[p] + r.w[wV + 1] * hv1[p];
-    Fo[p] = he * ue[p];
-    if (W::TR) {
-      qo[p] = (a0[p] + a1[p]) / 2;
-    } else {
-      const double z = r.w[wR] * a0[p] + r.w[wR + 1] * a1[p];
-      const double eta = r.w[wR] * hv0[p] + r.w[wR + 1] * hv1[p];
-      qo[p] = (z + r.w[W::FED - 1]) / eta;
-    }
+  double he;
+  if (KE == KE_CELL)
+    he = r.w[0] * hc0 + r.w[1] * hc1;
+  else if (KE == KE_VERTEX)
+    he = r.w[wV] * hv0 + r.w[wV + 1] * hv1;
+  else
+    he = r.w[0] * hc0 + r.w[1] * hc1 + r.w[wV] * hv0 + r.w[wV + 1] * hv1;
+  S.F[e] = he * ue;
+  if (W::TR) {
+    S.q[e] = (a0 + a1) / 2;
+  } else {
+    const double z = r.w[wR] * a0 + r.w[wR + 1] * a1;
+    const double eta = r.w[wR] * hv0 + r.w[wR + 1] * hv1;
+    S.q[e] = (z + r.w[W::FED - 1]) / eta;
   }
-  round_to<R, P>(Fo);
-  round_to<R, P>(qo);
-  st_members<double, P>(S.F + e * MC + mm, Fo);
-  st_members<double, P>(S.q + e * MC + mm, qo);
 }
 
 // cells: the Bernoulli function B
-template <int PV, int KE, class R, int MC, int P, class Vec>
+template <int PV, int KE, class Vec>
 __device__ __forceinline__ void patch_cell(const PatchRow<PatchRows<PV, KE>::FCI, PatchRows<PV, KE>::FCD>& r,
-                                           const Vec& S, double gravity, int i, int mm) {
+                                           const Vec& S, double gravity, int i) {
   using W = PatchRows<PV, KE>;
   constexpr int wV = W::CELL ? 6 : 0;
-  double hi[P], K[P], B[P];
-  ld_members<double, P>(S.h + i * MC + mm, hi);
-#pragma unroll
-  for (int p = 0; p < P; ++p) K[p] = 0.0;
+  double B = gravity * S.h[i];
   if (W::CELL) {
+    double K = 0.0;
 #pragma unroll
     for (int k = 0; k < CW; ++k) {
-      double x[P];
-      ld_members<double, P>(S.u + r.ix[k] * MC + mm, x);
-#pragma unroll
-      for (int p = 0; p < P; ++p) K[p] += r.w[k] * (x[p] * x[p]);
+      const double x = S.u[r.ix[k]];
+      K += r.w[k] * (x * x);
     }
+    B = K + B;
   }
-#pragma unroll
-  for (int p = 0; p < P; ++p) B[p] = W::CELL ? K[p] + gravity * hi[p] : gravity * hi[p];
   if (W::VERT) {
-    double s[P];
+    double s = 0.0;
 #pragma unroll
-    for (int p = 0; p < P; ++p) s[p] = 0.0;
-#pragma unroll
-    for (int k = 0; k < CW; ++k) {
-      double x[P];
-      ld_members<double, P>(S.v2 + r.ix[wV + k] * MC + mm, x);
-#pragma unroll
-      for (int p = 0; p < P; ++p) s[p] += r.w[wV + k] * x[p];
-    }
-#pragma unroll
-    for (int p = 0; p < P; ++p) B[p] += s[p];
+    for (int k = 0; k < CW; ++k) s += r.w[wV + k] * S.v2[r.ix[wV + k]];
+    B += s;
   }
-  round_to<R, P>(B);
-  st_members<double, P>(S.B + i * MC + mm, B);
+  S.B[i] = B;
 }
 
 // owned edges: du
-template <int PV, int KE, int MC, int P, class Vec>
-__device__ __forceinline__ void patch_du(const PatchRow<PatchRows<PV, KE>::TEI, PatchRows<PV, KE>::TED>& r,
-                                         const Vec& S, int e, int mm, double (&du)[P]) {
+template <int PV, int KE, class Vec>
+__device__ __forceinline__ double patch_du(const PatchRow<PatchRows<PV, KE>::TEI, PatchRows<PV, KE>::TED>& r,
+                                           const Vec& S, int e) {
   using W = PatchRows<PV, KE>;
   constexpr int C0 = 2 * W::TEI - 2;
-  double s[P], b0[P], b1[P];
-#pragma unroll
-  for (int p = 0; p < P; ++p) s[p] = 0.0;
+  double s = 0.0;
   if (W::TR) {
-    double qself[P];
-    ld_members<double, P>(S.q + e * MC + mm, qself);
+    const double qself = S.q[e];
 #pragma unroll
-    for (int k = 0; k < W::SW; ++k) {
-      double f[P], q[P];
-      ld_members<double, P>(S.F + r.ix[k] * MC + mm, f);
-      ld_members<double, P>(S.q + r.ix[k] * MC + mm, q);
-#pragma unroll
-      for (int p = 0; p < P; ++p) s[p] += r.w[k] * f[p] * (qself[p] + q[p]);
-    }
+    for (int k = 0; k < W::SW; ++k) s += r.w[k] * S.F[r.ix[k]] * (qself + S.q[r.ix[k]]);
+    s = s / 2;
   } else if (PV == PVM_GASSMANN_DERIVED) {
 #pragma unroll
     for (int b = 0; b < 2; ++b) {  // the two vertices' blocks of six
-      double qa[P], qb[P];
-      ld_members<double, P>(S.q + r.ix[6 * b] * MC + mm, qa);
-      ld_members<double, P>(S.q + r.ix[6 * b + 3] * MC + mm, qb);
+      const double qa = S.q[r.ix[6 * b]], qb = S.q[r.ix[6 * b + 3]];
 #pragma unroll
-      for (int k = 6 * b; k < 6 * b + 6; ++k) {
-        double f[P];
-        ld_members<double, P>(S.F + r.ix[k] * MC + mm, f);
-#pragma unroll
-        for (int p = 0; p < P; ++p) s[p] += r.w[k] * f[p] * (derived_pv_source(k) % 6 == 0 ? qa[p] : qb[p]);
-      }
+      for (int k = 6 * b; k < 6 * b + 6; ++k) s += r.w[k] * S.F[r.ix[k]] * (derived_pv_source(k) % 6 == 0 ? qa : qb);
     }
   } else {
-    double qself[P];
-    if (PV == PVM_GASSMANN_MEAN) ld_members<double, P>(S.q + e * MC + mm, qself);
+    const double qself = PV == PVM_GASSMANN_MEAN ? S.q[e] : 0.0;
 #pragma unroll
     for (int k = 0; k < W::SW; ++k) {
-      double f[P], q[P];
-      ld_members<double, P>(S.F + r.ix[k] * MC + mm, f);
-      ld_members<double, P>(S.q + r.ix[PV == PVM_GASSMANN ? W::SW + k : k] * MC + mm, q);
-#pragma unroll
-      for (int p = 0; p < P; ++p) s[p] += r.w[k] * f[p] * (PV == PVM_GASSMANN_MEAN ? (qself[p] + q[p]) / 2 : q[p]);
+      const double q = S.q[r.ix[PV == PVM_GASSMANN ? W::SW + k : k]];
+      s += r.w[k] * S.F[r.ix[k]] * (PV == PVM_GASSMANN_MEAN ? (qself + q) / 2 : q);
     }
   }
-  ld_members<double, P>(S.B + (r.ix[C0] & PATCH_INDEX) * MC + mm, b0);
-  ld_members<double, P>(S.B + r.ix[C0 + 1] * MC + mm, b1);
-#pragma unroll
-  for (int p = 0; p < P; ++p) du[p] = (W::TR ? s[p] / 2 : s[p]) - (b1[p] - b0[p]) * r.w[W::TED - 1];
+  return s - (S.B[r.ix[C0 + 1]] - S.B[r.ix[C0] & PATCH_INDEX]) * r.w[W::TED - 1];
 }
 
 // owned cells: dh
-template <int PV, int KE, int MC, int P, class Vec>
-__device__ __forceinline__ void patch_dh(const PatchRow<3, 6>& r, const Vec& S, int mm, double (&dh)[P]) {
-  double s[P];
+template <class Vec>
+__device__ __forceinline__ double patch_dh(const PatchRow<3, 6>& r, const Vec& S) {
+  double s = 0.0;
 #pragma unroll
-  for (int p = 0; p < P; ++p) s[p] = 0.0;
-#pragma unroll
-  for (int k = 0; k < CW; ++k) {
-    double f[P];
-    ld_members<double, P>(S.F + (k == 0 ? r.ix[k] & PATCH_INDEX : r.ix[k]) * MC + mm, f);
-#pragma unroll
-    for (int p = 0; p < P; ++p) s[p] += r.w[k] * f[p];
-  }
-#pragma unroll
-  for (int p = 0; p < P; ++p) dh[p] = -s[p];
+  for (int k = 0; k < CW; ++k) s += r.w[k] * S.F[k == 0 ? r.ix[k] & PATCH_INDEX : r.ix[k]];
+  return -s;
 }
 
 // One tendency of every patch (a block each), from the caller's state to the caller's tendency.
@@ -430,7 +309,7 @@ __global__ void __launch_bounds__(512, 2) k_patch_tendency(const PatchParams A) 
     reinterpret_cast<int*>(&D)[tid] = reinterpret_cast<const int*>(A.desc + blockIdx.x)[tid];
   __syncthreads();
   const PatchTab<false> T{A.tables + D.block};
-  using Vec = PatchVectors<PV, KE, 1, false>;
+  using Vec = PatchVectors<PV, KE, false>;
   const Vec S(patch_sm, D);
   const int vp = patch_pad(D.nLV), ep = patch_pad(D.nLE), cp = patch_pad(D.nLC), tp = patch_pad(D.nOE),
             op = patch_pad(D.nOC);
@@ -447,36 +326,32 @@ __global__ void __launch_bounds__(512, 2) k_patch_tendency(const PatchParams A) 
   for (int v = tid; v < D.nLV; v += nt) {
     PatchRow<W::VI, W::VD> r;
     r.load(T, D.vert, vp, v);
-    patch_vertex<PV, KE, double, 1, 1>(r, S, v, 0);
+    patch_vertex<PV, KE>(r, S, v);
   }
   __syncthreads();
   for (int i = tid; i < D.nLC; i += nt) {
     PatchRow<W::FCI, W::FCD> r;
     r.load(T, D.fcell, cp, i);
-    patch_cell<PV, KE, double, 1, 1>(r, S, A.gravity, i, 0);
+    patch_cell<PV, KE>(r, S, A.gravity, i);
   }
   if (W::CELL && !Vec::F_OWN) __syncthreads();
   for (int e = tid; e < D.nLE; e += nt) {
     PatchRow<W::FEI, W::FED> r;
     r.load(T, D.fedge, ep, e);
-    patch_edge<PV, KE, double, 1, 1>(r, S, e, 0);
+    patch_edge<PV, KE>(r, S, e);
   }
   __syncthreads();
   for (int e = tid; e < D.nOE; e += nt) {
     PatchRow<W::TEI, W::TED> r;
     r.load(T, D.tedge, tp, e);
-    double du[1];
-    patch_du<PV, KE, 1, 1>(r, S, e, 0, du);
     const int g = D.e0 + e;
-    A.dy[A.map ? A.map[g] : g] = du[0];
+    A.dy[A.map ? A.map[g] : g] = patch_du<PV, KE>(r, S, e);
   }
   for (int i = tid; i < D.nOC; i += nt) {
     PatchRow<3, 6> r;
     r.load(T, D.tcell, op, i);
-    double dh[1];
-    patch_dh<PV, KE, 1, 1>(r, S, 0, dh);
     const int g = A.ne + D.c0 + i;
-    A.dy[A.map ? A.map[g] : g] = dh[0];
+    A.dy[A.map ? A.map[g] : g] = patch_dh(r, S);
   }
 }
 
@@ -504,7 +379,7 @@ __global__ void __launch_bounds__(512, 1) k_patch_rk4(const PatchParams A) {
   const int nHE = D.nSE - D.nOE, nH = nHE + D.nSC - D.nOC, nO = D.nOE + D.nOC;
   double* ykept = reinterpret_cast<double*>(kept + D.bytes);  // y of the owned edges and cells
   double* akept = ykept + nO;                                 // their accumulator
-  const PatchVectors<PV, KE, 1, true> S(akept + nO, D);
+  const PatchVectors<PV, KE, true> S(akept + nO, D);
   const int vp = patch_pad(D.nLV), ep = patch_pad(D.nLE), cp = patch_pad(D.nLC), tp = patch_pad(D.nOE),
             op = patch_pad(D.nOC);
   const double half = A.dt / 2, sixth = A.dt / 6;
@@ -539,45 +414,45 @@ __global__ void __launch_bounds__(512, 1) k_patch_rk4(const PatchParams A) {
       for (int v = tid; v < D.nLV; v += nt) {
         PatchRow<W::VI, W::VD> r;
         r.load(T, D.vert, vp, v);
-        patch_vertex<PV, KE, double, 1, 1>(r, S, v, 0);
+        patch_vertex<PV, KE>(r, S, v);
       }
       __syncthreads();
       for (int e = tid; e < D.nLE; e += nt) {
         PatchRow<W::FEI, W::FED> r;
         r.load(T, D.fedge, ep, e);
-        patch_edge<PV, KE, double, 1, 1>(r, S, e, 0);
+        patch_edge<PV, KE>(r, S, e);
       }
       for (int i = nt - 1 - tid; i < D.nLC; i += nt) {  // from the last thread down: the first have more edges
         PatchRow<W::FCI, W::FCD> r;
         r.load(T, D.fcell, cp, i);
-        patch_cell<PV, KE, double, 1, 1>(r, S, A.gravity, i, 0);
+        patch_cell<PV, KE>(r, S, A.gravity, i);
       }
       __syncthreads();
       const double c = stage == EPI_STAGE3 ? A.dt : half;
       Tagged* out = A.exchange + (size_t)((version + 1u) & 1u) * A.N;
       for (int j = tid; j < nO; j += nt) {
-        double kv[1], next;
+        double kv, next;
         bool shared;
         if (j < D.nOE) {
           PatchRow<W::TEI, W::TED> r;
           r.load(T, D.tedge, tp, j);
-          patch_du<PV, KE, 1, 1>(r, S, j, 0, kv);
+          kv = patch_du<PV, KE>(r, S, j);
           shared = (r.ix[2 * W::TEI - 2] & PATCH_PUBLISH) != 0;
         } else {
           PatchRow<3, 6> r;
           r.load(T, D.tcell, op, j - D.nOE);
-          patch_dh<PV, KE, 1, 1>(r, S, 0, kv);
+          kv = patch_dh(r, S);
           shared = (r.ix[0] & PATCH_PUBLISH) != 0;
         }
         const double y = ykept[j];
         if (stage == EPI_STAGE4) {
-          next = y + sixth * (akept[j] + kv[0]);
+          next = y + sixth * (akept[j] + kv);
           if (!isfinite(next)) atomicOr(A.nonfinite, 1);
           ykept[j] = next;
           if (step == A.nsteps - 1) A.y[global(j)] = next;
         } else {
-          akept[j] = stage == EPI_STAGE1 ? kv[0] : akept[j] + 2 * kv[0];
-          next = y + c * kv[0];
+          akept[j] = stage == EPI_STAGE1 ? kv : akept[j] + 2 * kv;
+          next = y + c * kv;
         }
         if (shared) publish(out + global(j), next, version + 1u);
         *slot(j) = next;  // no phase reads the stage state any more
