@@ -248,10 +248,13 @@ __device__ __forceinline__ uint4 half_bf16x8(const __nv_bfloat16* p) {
   for (int k = 0; k < 4; ++k) h[k] = __hmul2(h[k], half);
   return q;
 }
-// x as the sum of three BF16 values (3 x 8 significant bits: exact), in columns 0..2 of a chunk row
+// x as the sum of three BF16 values (3 x 8 significant bits: exact), in columns 0..2 of a chunk row.
+// A finite x that would round to infinity takes the largest BF16 value first; an infinite x is its
+// first term alone (infinity less infinity would be NaN).
 __device__ __forceinline__ uint4 split_bf16(float x) {
-  const __nv_bfloat16 hi = __float2bfloat16_rn(x);
-  const float r1 = x - __bfloat162float(hi);
+  __nv_bfloat16 hi = __float2bfloat16_rn(x);
+  if (isinf(__bfloat162float(hi))) hi = __float2bfloat16_rz(x);
+  const float r1 = isinf(x) ? 0.0f : x - __bfloat162float(hi);
   const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
   const __nv_bfloat16 lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
   const uint32_t h = *reinterpret_cast<const uint16_t*>(&hi), m = *reinterpret_cast<const uint16_t*>(&mid),

@@ -107,6 +107,24 @@ def test_biases_and_ragged_rows_match_oracle(require_gpu, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("layer", ["b1", "b2"])
+def test_infinite_bias_saturates_its_unit(require_gpu, layer):
+    """An infinite bias gives its unit's activation as FP32 addition does: gelu(inf) = inf, so with
+    weights of one sign both outputs are infinite, never NaN."""
+    import torch
+    import dmplex_b200.closure as cl
+    p = co.unpack(co.init_params(11))
+    for name in ("W1", "W2", "W3"):
+        p[name] = np.abs(p[name])
+    p["W3"][1] *= -1
+    p[layer][5] = np.inf
+    X = np.abs(_data(200, 1)[0])
+    Xd = torch.from_numpy(X.astype(np.float32)).to(torch.bfloat16).cuda().contiguous()
+    Y = cl.ClosureMLP(co.pack(p).astype(np.float32)).forward(Xd).cpu().numpy()
+    assert np.all(Y[:, 0] == np.inf) and np.all(Y[:, 1] == -np.inf)
+
+
+@pytest.mark.gpu
 def test_training_reduces_loss(require_gpu):
     import torch
     import dmplex_b200.closure as cl
