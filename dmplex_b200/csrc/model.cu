@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "model.hpp"
+#include "pointers.hpp"
 
 using trisk::Error;
 
@@ -91,6 +92,16 @@ bool is_device_pointer(const void* p) {
     return false;
   }
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+}
+
+bool is_kernel_accessible(const void* p, int device) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const bool managed = a.type == cudaMemoryTypeManaged;
+  return (a.type == cudaMemoryTypeDevice || managed) && kernel_can_access(p, managed, a.device, device);
 }
 
 void launch_gather(cudaStream_t stream, double* dst, const double* src, const int32_t* idx, int64_t n) {
@@ -1043,7 +1054,7 @@ int trisk_tendency(TriskModel* model, const double* y, double* dy) {
   if (!y || !dy) throw Error(TRISK_ERR_ARGUMENT, "NULL state");
   DeviceGuard guard(m.device);
   const bool apart = y + m.N <= dy || dy + m.N <= y;
-  if (m.patches.n && apart && is_device_pointer(y) && is_device_pointer(dy)) {
+  if (m.patches.n && apart && is_kernel_accessible(y, m.device) && is_kernel_accessible(dy, m.device)) {
     // one launch, straight from the caller's state to the caller's tendency
     order_after_caller(m.stream, m.caller_ev);
     patch_tendency(m, y, dy, m.identity ? nullptr : m.state_n2o);

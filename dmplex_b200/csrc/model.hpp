@@ -38,6 +38,8 @@ struct DeviceGuard {
 
 // true for device or managed memory, false for host memory (pageable or pinned)
 bool is_device_pointer(const void* p);
+// true for such memory that a kernel on `device` may dereference as doubles (pointers.hpp)
+bool is_kernel_accessible(const void* p, int device);
 // Orders `stream` after all work queued so far on the legacy default stream (and, by its
 // semantics, on every blocking stream), so a caller's device buffer filled or still read on
 // those streams (PyTorch's default stream among them) is safe to use from `stream`.

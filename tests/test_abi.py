@@ -88,3 +88,25 @@ def test_tables_are_deterministic():
     for k, v in a.items():
         if isinstance(v, np.ndarray):
             assert np.array_equal(v, b[k]), k
+
+
+def test_which_pointers_a_kernel_may_access(tmp_path):
+    """csrc/pointers.hpp, compiled alone: aligned memory of the model's device and aligned managed
+    memory of any; another device's memory and other byte addresses are left to the copy engine."""
+    import subprocess
+    source = tmp_path / "rule.cpp"
+    source.write_text("""
+#include <cstdio>
+#include "pointers.hpp"
+int main() {
+  for (long address = 4096; address <= 4100; address += 4)
+    for (int managed = 0; managed < 2; ++managed)
+      for (int device = 0; device < 2; ++device)
+        std::putchar('0' + trisk::kernel_can_access(reinterpret_cast<void*>(address), managed, device, 0));
+}
+""")
+    exe = str(tmp_path / "rule")
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", os.path.join(ROOT, "dmplex_b200", "csrc"),
+                    str(source), "-o", exe], check=True)
+    out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout
+    assert out == "1011" + "0000"  # [own, other] device memory, then managed; unaligned: never

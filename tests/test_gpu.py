@@ -369,3 +369,21 @@ def test_patches_bitwise(require_gpu, n, pv, ke, reorder):
     assert m.launch_count() - before <= 3
     o.rk4_step(ref, dt, 8)
     assert np.array_equal(a, ref)
+
+
+@pytest.mark.parametrize("offset", [4, 8])
+def test_tendency_of_a_state_at_any_byte_address(require_gpu, offset):
+    """A model in file numbering copies the caller's device state, so it takes one at any byte
+    address (and of any device); only states a kernel can dereference skip the copy."""
+    import torch
+    from dmplex_b200 import _lib
+    g = trisk_grid(2)
+    m = d.TRiSKShallowWater(g, reorder=False)
+    y = perturbed_tc2(g)
+    expect = np.zeros_like(y)
+    d.tendency(expect, y, m)
+    state = torch.zeros(y.nbytes + 16, dtype=torch.uint8, device="cuda")
+    out = torch.zeros_like(state)
+    state[offset:offset + y.nbytes] = torch.from_numpy(y.view(np.uint8)).cuda()
+    _lib.check(_lib.lib.trisk_tendency(m.handle, state.data_ptr() + offset, out.data_ptr() + offset))
+    assert np.array_equal(out[offset:offset + y.nbytes].cpu().numpy().view(np.float64), expect)
