@@ -1215,6 +1215,7 @@ int trisk_autotune(TriskModel* model, double* y, double dt, int32_t steps, doubl
   // one was set, is left off.
   m.persistent = false;
   m.use_patches = false;
+  m.patches_held = false;
   static const int choices[] = {64, 128, 256};
   static const int keep_mb[] = {0, 8, 16, 24, 32, 40, 48, 64};
   cudaEvent_t e0, e1;
@@ -1333,6 +1334,7 @@ int trisk_model_set_block(TriskModel* model, const int32_t block[3]) {
   CUDA_CHECK(cudaStreamSynchronize(m.stream));
   for (int p = 0; p < 3; ++p) m.block[p] = block[p];
   m.use_patches = false;  // the blocks are the three-launch tendency's
+  m.patches_held = false;
   if (m.graph) {  // recaptured with the new launch shapes at the next step
     cudaGraphExecDestroy(m.graph);
     m.graph = nullptr;
@@ -1380,7 +1382,13 @@ int trisk_model_set_l2_residency(TriskModel* model, int64_t bytes, int32_t windo
     if (limit < keep) CUDA_CHECK(cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, keep));
   }
   m.l2_keep_bytes = keep;
-  m.use_patches = false;  // the table block is the three-launch tendency's
+  if (keep > 0) {  // the table block is the three-launch tendency's ...
+    m.patches_held |= m.use_patches;
+    m.use_patches = false;
+  } else {  // ... until it is given up
+    m.use_patches |= m.patches_held;
+    m.patches_held = false;
+  }
   m.l2_window = win && keep > 0;
   m.T.keep_end = keep ? m.table_base + keep : nullptr;
   if (m.graph) {  // recaptured with the new table pointers and launch attributes

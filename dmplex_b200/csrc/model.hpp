@@ -86,6 +86,7 @@ struct TriskModel {
   int* barrier_err = nullptr;            // a grid-barrier wait gave up
   trisk::PatchSet patches;               // whole tendencies and RK4 runs from shared memory (patch.hpp)
   bool use_patches = false;              // for the RK4 runs; an explicit choice of launches turns it off
+  bool patches_held = false;             // turned off for as long as an L2-resident prefix is set
   trisk::Coefficients C;  // file numbering, 0-based (kept for export)
   CoefficientExport exported;
   std::vector<int32_t> cell_n2o, edge_n2o, vert_n2o, cell_o2n, edge_o2n, vert_o2n;

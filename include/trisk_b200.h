@@ -246,7 +246,7 @@ int trisk_model_set_block(TriskModel* model, const int32_t block[3]);
 int trisk_model_set_persistent(TriskModel* model, int32_t on);
 int trisk_model_get_persistent(TriskModel* model, int32_t* on);
 /* L2 residency of the tables (no reference counterpart; the three-launch phases', which RK4
- * steps use from then on). The first `bytes` of the model's
+ * steps use while bytes > 0 is set). The first `bytes` of the model's
  * packed table block (the tendency phase's tables first, then the flux phase's, then the
  * vertex phase's) are loaded with an L2 evict-last policy, so they stay in L2 from one
  * phase launch and one RK4 stage to the next instead of streaming from HBM; with window = 1

@@ -387,3 +387,30 @@ def test_tendency_of_a_state_at_any_byte_address(require_gpu, offset):
     state[offset:offset + y.nbytes] = torch.from_numpy(y.view(np.uint8)).cuda()
     _lib.check(_lib.lib.trisk_tendency(m.handle, state.data_ptr() + offset, out.data_ptr() + offset))
     assert np.array_equal(out[offset:offset + y.nbytes].cpu().numpy().view(np.float64), expect)
+
+
+def test_l2_residency_of_zero_gives_the_patches_back(require_gpu):
+    """A prefix of L2-resident tables keeps RK4 runs on the launches that read them; setting it back
+    to none is the default again, except where the launches' blocks were chosen too."""
+    g = trisk_grid(4)
+    m = d.TRiSKShallowWater(g)
+    y = tc2_state(g)
+
+    def launches():
+        before = m.launch_count()
+        d.rk4_step(y, 0.01, d.tendency, d.RK4Cache(y), m, nsteps=5)
+        return m.launch_count() - before
+
+    default, phases = launches(), 5 * 12 + 2
+    assert default < phases
+    m.set_l2_residency(0)
+    assert launches() == default
+    m.set_l2_residency(1 << 20)
+    m.set_l2_residency(2 << 20)
+    assert launches() == phases
+    m.set_l2_residency(0)
+    assert launches() == default
+    m.set_l2_residency(1 << 20)
+    m.set_block([128, 128, 128])
+    m.set_l2_residency(0)
+    assert launches() == phases
