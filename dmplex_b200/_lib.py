@@ -162,6 +162,7 @@ def _load():
         "trisk_diagnostics": (C.c_int, [_p, _p, _p, _p, _p]),
         "trisk_relative_vorticity": (C.c_int, [_p, _p, _p]),
         "trisk_model_stream": (C.c_int, [_p, C.POINTER(_p)]),
+        "trisk_model_expire_wait_once": (C.c_int, [_p]),
         "trisk_launch_count": (_i64, [_p]),
         "trisk_model_bytes": (C.c_int, [_p, _p]),
         "trisk_profile_phases": (C.c_int, [_p, _p, _f64, _i64, _p]),

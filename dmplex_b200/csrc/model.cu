@@ -1398,6 +1398,15 @@ int trisk_model_set_l2_residency(TriskModel* model, int64_t bytes, int32_t windo
   TRISK_API_END
 }
 
+int trisk_model_expire_wait_once(TriskModel* model) {
+  TRISK_API_BEGIN
+  TriskModel& m = *checked(model);
+  if (!m.patches.runs || m.patches.n < 2)
+    throw Error(TRISK_ERR_UNSUPPORTED, "the model's RK4 runs have no blocks that wait for one another");
+  m.patches.expire = true;
+  TRISK_API_END
+}
+
 int trisk_profile_phases(TriskModel* model, double* y, double dt, int64_t nsteps, double ms[3]) {
   TRISK_API_BEGIN
   TriskModel& m = *checked(model);

@@ -370,6 +370,9 @@ namespace {
 // Dynamic shared memory of a block with an SM to itself (227 KB less its static part).
 constexpr size_t PATCH_SMEM = 225 * 1024;
 constexpr int PATCH_STEPS = 4096;  // RK4 steps a launch
+// A wait for a neighbour's value takes microseconds; a neighbour may have to wait for an SM that
+// another stream's kernel holds. A run that tests the wait gives up sooner.
+constexpr long long PATCH_WAIT_NS = 10000000000LL, PATCH_TEST_WAIT_NS = 5000000LL;
 
 template <int PV, int KE>
 const void* rk4_kernel() {
@@ -462,6 +465,9 @@ void patch_rk4(TriskModel& m, double dt, int64_t nsteps) {
   PatchSet& S = m.patches;
   PatchParams A = params(m);
   A.dt = dt;
+  A.wait_ns = S.expire ? PATCH_TEST_WAIT_NS : PATCH_WAIT_NS;
+  A.silent = S.expire ? 0 : -1;
+  S.expire = false;
   for (int64_t left = nsteps; left > 0; left -= A.nsteps) {
     A.nsteps = (int)std::min<int64_t>(left, PATCH_STEPS);
     A.base = S.base;

@@ -40,6 +40,8 @@ struct PatchParams {
   double dt;
   int nsteps;
   unsigned base;        // the version of the state in y
+  long long wait_ns;    // the longest wait for a neighbour's value
+  int silent;           // a patch that publishes nothing (a test of that wait), or -1
 };
 
 // A patch's table block, in global memory (read past L1) or in shared memory.
@@ -114,10 +116,9 @@ __device__ __forceinline__ void publish(Tagged* p, double x, unsigned version) {
   asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"((b & 0xFFFFFFFFull) | t), "l"((b >> 32) | t)
                : "memory");
 }
-// The value of `version` at p, waited for; false if the wait gave up: after ten seconds (or 2^31
-// polls, which the clock always beats; a neighbour may have to wait for an SM that another
-// stream's kernel holds), or when another block's has.
-__device__ __forceinline__ bool receive(const Tagged* p, unsigned version, double& x, int* err) {
+// The value of `version` at p, waited for; false if the wait gave up: after wait_ns (or 2^31 polls,
+// which the clock always beats), or when another block's has.
+__device__ __forceinline__ bool receive(const Tagged* p, unsigned version, double& x, int* err, long long wait_ns) {
   long long start = 0;
   for (unsigned i = 1;; ++i) {
     unsigned long long lo, hi;
@@ -129,7 +130,7 @@ __device__ __forceinline__ bool receive(const Tagged* p, unsigned version, doubl
     if ((i & 255u) == 0) {
       const long long now = barrier_ns();
       if (start == 0) start = now;
-      if (now - start > 10000000000LL || *reinterpret_cast<volatile int*>(err) != 0 || i >= (1u << 31)) {
+      if (now - start > wait_ns || *reinterpret_cast<volatile int*>(err) != 0 || i >= (1u << 31)) {
         atomicExch(err, 1);
         x = 0.0;
         return false;
@@ -405,7 +406,7 @@ __global__ void __launch_bounds__(512, 1) k_patch_rk4(const PatchParams A) {
         if (step == 0 && stage == EPI_STAGE1)
           x = __ldcg(A.y + g);
         else
-          ok &= receive(A.exchange + (size_t)(version & 1u) * A.N + g, version, x, A.err) ? 1 : 0;
+          ok &= receive(A.exchange + (size_t)(version & 1u) * A.N + g, version, x, A.err, A.wait_ns) ? 1 : 0;
         (edge ? S.u[D.nOE + i] : S.h[D.nOC + i]) = x;
       }
       if (!ok) gave_up = 1;
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(512, 1) k_patch_rk4(const PatchParams A) {
           akept[j] = stage == EPI_STAGE1 ? kv : akept[j] + 2 * kv;
           next = y + c * kv;
         }
-        if (shared) publish(out + global(j), next, version + 1u);
+        if (shared && (int)blockIdx.x != A.silent) publish(out + global(j), next, version + 1u);
         *slot(j) = next;  // no phase reads the stage state any more
       }
     }

@@ -44,6 +44,7 @@ struct PatchSet {
   Tagged* exchange = nullptr;  // the halos' published values
   int* err = nullptr;          // a wait for a neighbour gave up
   unsigned base = 0;           // version of the state between calls
+  bool expire = false;         // the next run tests the bounded wait (trisk_model_expire_wait_once)
 };
 
 // Decomposes the mesh into `patches` runs of cells (host side only); false if the edges are not

@@ -161,6 +161,11 @@ class TRiSKShallowWater:
         that stay in L2), or as the CUDA graph of twelve launches per step."""
         check(lib.trisk_model_set_persistent(self._h, int(bool(on))))
 
+    def expire_wait_once(self) -> None:
+        """Test of the bounded wait: one block of the next RK4 run from shared memory hands its
+        neighbours nothing, so the run gives up and its call raises TriskError."""
+        check(lib.trisk_model_expire_wait_once(self._h))
+
     def set_l2_residency(self, nbytes: int, window: bool = False) -> None:
         """Keeps the first nbytes of the packed tables in L2 (evict-last loads; with window
         also a persisting access-policy window). 0 streams every table."""

@@ -245,6 +245,12 @@ int trisk_model_set_block(TriskModel* model, const int32_t block[3]);
  * returns TRISK_ERR_TIMEOUT. TRISK_ERR_UNSUPPORTED without cooperative launch. */
 int trisk_model_set_persistent(TriskModel* model, int32_t on);
 int trisk_model_get_persistent(TriskModel* model, int32_t* on);
+/* Test of the bounded wait (no reference counterpart): in this model's next RK4 run from shared
+ * memory one block hands its neighbours nothing, so their waits run out after a few milliseconds and
+ * the run reports TRISK_ERR_TIMEOUT at the next synchronizing call; the state is then unspecified.
+ * The model stays usable and later runs are unaffected. TRISK_ERR_UNSUPPORTED for a model without
+ * such runs. */
+int trisk_model_expire_wait_once(TriskModel* model);
 /* L2 residency of the tables (no reference counterpart; the three-launch phases', which RK4
  * steps use while bytes > 0 is set). The first `bytes` of the model's
  * packed table block (the tendency phase's tables first, then the flux phase's, then the

@@ -414,3 +414,29 @@ def test_l2_residency_of_zero_gives_the_patches_back(require_gpu):
     m.set_block([128, 128, 128])
     m.set_l2_residency(0)
     assert launches() == phases
+
+
+@pytest.mark.parametrize("n", [1, 5])
+def test_patch_wait_gives_up_and_the_model_stays_usable(require_gpu, n):
+    """A wait for a neighbouring patch that runs out (here: one patch publishes nothing) ends the run
+    with TRISK_ERR_TIMEOUT after a few milliseconds, from the smallest exchange to a patch on every SM;
+    the next runs are the launches' again, bit for bit."""
+    g = trisk_grid(n)
+    si = w.si_parameters()
+    m = d.TRiSKShallowWater(g, **si)
+    phases = d.TRiSKShallowWater(g, block=128, **si)
+    dt = w.courant_dt(g, 0.1)
+    a = w.synthetic_state(g, seed=6)
+    b = a.copy()
+    d.rk4_step(a, dt, d.tendency, d.RK4Cache(a), m, nsteps=9)
+    lost = a.copy()
+    m.expire_wait_once()
+    with pytest.raises(d.TriskError) as err:
+        d.rk4_step(lost, dt, d.tendency, d.RK4Cache(lost), m, nsteps=20)
+    assert err.value.status == 5
+    d.rk4_step(a, dt, d.tendency, d.RK4Cache(a), m, nsteps=10)
+    d.rk4_step(b, dt, d.tendency, d.RK4Cache(b), phases, nsteps=19)
+    assert np.array_equal(a, b)
+    with pytest.raises(d.TriskError) as err:  # no patches: nothing waits
+        d.TRiSKShallowWater(trisk_grid(6)).expire_wait_once()
+    assert err.value.status == 6
