@@ -432,17 +432,17 @@ void check_flag(TriskModel& m) {
   CUDA_CHECK(cudaMemcpyAsync(flags, m.flag, sizeof(flags), cudaMemcpyDeviceToHost, m.stream));
   if (m.barrier_err) CUDA_CHECK(cudaMemcpyAsync(&err, m.barrier_err, sizeof(int), cudaMemcpyDeviceToHost, m.stream));
   CUDA_CHECK(cudaStreamSynchronize(m.stream));
-  patch_check(m, flags[1]);
+  // every mark goes before the first is reported: none is left for the next call
+  if (flags[0] || flags[1]) CUDA_CHECK(cudaMemsetAsync(m.flag, 0, sizeof(flags), m.stream));
+  if (flags[1]) patch_restart(m);
   if (err) {
     CUDA_CHECK(cudaMemsetAsync(m.barrier, 0, 2 * sizeof(unsigned), m.stream));
     CUDA_CHECK(cudaMemsetAsync(m.barrier_err, 0, sizeof(int), m.stream));
-    CUDA_CHECK(cudaStreamSynchronize(m.stream));
-    throw Error(TRISK_ERR_TIMEOUT, "a grid-barrier wait of the one-launch RK4 step gave up");
   }
-  if (flags[0]) {
-    CUDA_CHECK(cudaMemsetAsync(m.flag, 0, sizeof(int), m.stream));
-    throw Error(TRISK_ERR_NONFINITE, "the state became non-finite");
-  }
+  if (flags[1] || err) CUDA_CHECK(cudaStreamSynchronize(m.stream));
+  if (flags[1]) throw Error(TRISK_ERR_TIMEOUT, "a wait for a neighbouring patch gave up");
+  if (err) throw Error(TRISK_ERR_TIMEOUT, "a grid-barrier wait of the one-launch RK4 step gave up");
+  if (flags[0]) throw Error(TRISK_ERR_NONFINITE, "the state became non-finite");
 }
 
 // ---------------------------------------------------------------------------------------

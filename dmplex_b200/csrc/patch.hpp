@@ -57,7 +57,7 @@ void choose_patches(TriskModel& m);
 void patch_tendency(TriskModel& m, const double* y, double* dy, const int32_t* map);
 // nsteps RK4 steps of the internal state m.y in one cooperative launch.
 void patch_rk4(TriskModel& m, double dt, int64_t nsteps);
-// Throws TRISK_ERR_TIMEOUT if a wait gave up in the last run (the flags start again).
-void patch_check(TriskModel& m, int err);
+// The exchanged versions start again, after a run in which a wait gave up.
+void patch_restart(TriskModel& m);
 
 }  // namespace trisk

@@ -440,3 +440,25 @@ def test_patch_wait_gives_up_and_the_model_stays_usable(require_gpu, n):
     with pytest.raises(d.TriskError) as err:  # no patches: nothing waits
         d.TRiSKShallowWater(trisk_grid(6)).expire_wait_once()
     assert err.value.status == 6
+
+
+def test_timeout_leaves_no_mark_for_the_next_call(require_gpu):
+    """Of a non-finite state and a wait that gave up before the same synchronizing call the time-out
+    is reported, and neither is reported again."""
+    import torch
+    g = trisk_grid(4)
+    si = w.si_parameters()
+    m = d.TRiSKShallowWater(g, **si)
+    dt = w.courant_dt(g, 0.1)
+    y = w.synthetic_state(g, seed=6)
+    bad = y.copy()
+    bad[5] = np.nan
+    bad, lost = torch.from_numpy(bad).cuda(), torch.from_numpy(y).cuda()
+    m.rk4_async(bad, dt, 9)
+    m.expire_wait_once()
+    m.rk4_async(lost, dt, 20)
+    with pytest.raises(d.TriskError) as err:
+        m.synchronize()
+    assert err.value.status == 5
+    d.rk4_step(y, dt, d.tendency, d.RK4Cache(y), m, nsteps=9)
+    assert np.isfinite(y).all()
