@@ -293,10 +293,14 @@ void run_persistent(TriskModel& m, double dt, int64_t nsteps) {
   }
 }
 
+bool patches_take(const TriskModel& m, int64_t nsteps) {
+  return m.nc >= PATCH_RK4_MIN_CELLS || nsteps >= PATCH_RUN_STEPS;
+}
+
 void run_steps(TriskModel& m, double dt, int64_t nsteps) {
   if (m.persistent) {
     run_persistent(m, dt, nsteps);
-  } else if (m.use_patches && (m.nc >= PATCH_RK4_MIN_CELLS || nsteps >= PATCH_RUN_STEPS)) {
+  } else if (m.use_patches && patches_take(m, nsteps)) {
     patch_rk4(m, dt, nsteps);
   } else if (m.use_graph) {
     ensure_graph(m, dt);
@@ -427,23 +431,34 @@ void state_out(TriskModel& m, double* y_user, const double* src) {
   }
 }
 
-void check_flag(TriskModel& m) {
-  int flags[2] = {0, 0}, err = 0;  // a non-finite state, a patch's wait that gave up
-  CUDA_CHECK(cudaMemcpyAsync(flags, m.flag, sizeof(flags), cudaMemcpyDeviceToHost, m.stream));
-  if (m.barrier_err) CUDA_CHECK(cudaMemcpyAsync(&err, m.barrier_err, sizeof(int), cudaMemcpyDeviceToHost, m.stream));
+// What the runs so far have marked. Every mark goes before the first is reported: none is left for
+// the next call.
+struct Marks {
+  int nonfinite = 0, patch = 0;  // in this order in m.flag
+  int barrier = 0;
+};
+Marks take_marks(TriskModel& m) {
+  Marks k;
+  CUDA_CHECK(cudaMemcpyAsync(&k, m.flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, m.stream));
+  if (m.barrier_err)
+    CUDA_CHECK(cudaMemcpyAsync(&k.barrier, m.barrier_err, sizeof(int), cudaMemcpyDeviceToHost, m.stream));
   CUDA_CHECK(cudaStreamSynchronize(m.stream));
-  // every mark goes before the first is reported: none is left for the next call
-  if (flags[0] || flags[1]) CUDA_CHECK(cudaMemsetAsync(m.flag, 0, sizeof(flags), m.stream));
-  if (flags[1]) patch_restart(m);
-  if (err) {
+  if (k.nonfinite || k.patch) CUDA_CHECK(cudaMemsetAsync(m.flag, 0, 2 * sizeof(int), m.stream));
+  if (k.patch) patch_restart(m);
+  if (k.barrier) {
     CUDA_CHECK(cudaMemsetAsync(m.barrier, 0, 2 * sizeof(unsigned), m.stream));
     CUDA_CHECK(cudaMemsetAsync(m.barrier_err, 0, sizeof(int), m.stream));
   }
-  if (flags[1] || err) CUDA_CHECK(cudaStreamSynchronize(m.stream));
-  if (flags[1]) throw Error(TRISK_ERR_TIMEOUT, "a wait for a neighbouring patch gave up");
-  if (err) throw Error(TRISK_ERR_TIMEOUT, "a grid-barrier wait of the one-launch RK4 step gave up");
-  if (flags[0]) throw Error(TRISK_ERR_NONFINITE, "the state became non-finite");
+  if (k.patch || k.barrier) CUDA_CHECK(cudaStreamSynchronize(m.stream));
+  return k;
 }
+
+void report(const Marks& k) {
+  if (k.patch) throw Error(TRISK_ERR_TIMEOUT, "a wait for a neighbouring patch gave up");
+  if (k.barrier) throw Error(TRISK_ERR_TIMEOUT, "a grid-barrier wait of the one-launch RK4 step gave up");
+  if (k.nonfinite) throw Error(TRISK_ERR_NONFINITE, "the state became non-finite");
+}
+void check_flag(TriskModel& m) { report(take_marks(m)); }
 
 // ---------------------------------------------------------------------------------------
 // model construction
@@ -1209,18 +1224,24 @@ int trisk_autotune(TriskModel* model, double* y, double dt, int32_t steps, doubl
   if (!is_device_pointer(y)) throw Error(TRISK_ERR_ARGUMENT, "trisk_autotune needs a device state");
   // Times `steps` RK4 steps (graph + PDL as configured) for every combination of the three
   // phase block sizes, then for L2-resident table prefixes of several sizes with the best
-  // blocks, then the blocks again with the best prefix, and for meshes that fit half the L2
-  // the one-launch step, and keeps the fastest. Every candidate computes the same numbers;
-  // the state is restored from the caller's copy before each trial. A persisting window, if
-  // one was set, is left off.
+  // blocks, then the blocks again with the best prefix, for meshes that fit half the L2 the
+  // one-launch step, and the patches where a run of `steps` takes them, and keeps the fastest.
+  // Every candidate computes the same numbers; the state is restored from the caller's copy
+  // before each trial. A persisting window, if one was set, is left off.
+  Marks earlier = take_marks(m);
+  earlier.nonfinite = 0;
+  report(earlier);
+  const bool had_patches = m.use_patches || m.patches_held;
   m.persistent = false;
   m.use_patches = false;
   m.patches_held = false;
   static const int choices[] = {64, 128, 256};
   static const int keep_mb[] = {0, 8, 16, 24, 32, 40, 48, 64};
-  cudaEvent_t e0, e1;
-  CUDA_CHECK(cudaEventCreate(&e0));
-  CUDA_CHECK(cudaEventCreate(&e1));
+  struct Event {
+    cudaEvent_t e = nullptr;
+    Event() { CUDA_CHECK(cudaEventCreate(&e)); }
+    ~Event() { cudaEventDestroy(e); }
+  } e0, e1;
   int l2 = 0;
   CUDA_CHECK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, m.device));
   int best[3] = {m.block[0], m.block[1], m.block[2]};
@@ -1238,13 +1259,13 @@ int trisk_autotune(TriskModel* model, double* y, double dt, int32_t steps, doubl
       m.graph = nullptr;
     }
     state_in(m, y, m.y);
-    run_steps(m, dt, 2);  // warm-up (and graph capture)
-    CUDA_CHECK(cudaEventRecord(e0, m.stream));
+    run_steps(m, dt, m.use_patches ? steps : 2);  // warm-up (and graph capture)
+    CUDA_CHECK(cudaEventRecord(e0.e, m.stream));
     run_steps(m, dt, steps);
-    CUDA_CHECK(cudaEventRecord(e1, m.stream));
-    CUDA_CHECK(cudaEventSynchronize(e1));
+    CUDA_CHECK(cudaEventRecord(e1.e, m.stream));
+    CUDA_CHECK(cudaEventSynchronize(e1.e));
     float ms = 0;
-    CUDA_CHECK(cudaEventElapsedTime(&ms, e0, e1));
+    CUDA_CHECK(cudaEventElapsedTime(&ms, e0.e, e1.e));
     if (ms < best_t) {
       best_t = ms;
       best[0] = a;
@@ -1258,6 +1279,15 @@ int trisk_autotune(TriskModel* model, double* y, double dt, int32_t steps, doubl
       for (int b : choices)
         for (int c : choices) trial(a, b, c, keep);
   };
+  // A trial of a cooperative run: true if it is the fastest so far and no wait in it gave up.
+  auto faster = [&]() {
+    const double before = best_t;
+    trial(best[0], best[1], best[2], best_keep);  // the blocks and the prefix do not apply to it
+    const Marks k = take_marks(m);
+    if (k.patch || k.barrier) best_t = before;
+    return best_t < before;
+  };
+  bool use_persistent = false, use_patches = had_patches;
   try {
     blocks_pass(0);
     const int b0 = best[0], b1 = best[1], b2 = best[2];
@@ -1267,38 +1297,28 @@ int trisk_autotune(TriskModel* model, double* y, double dt, int32_t steps, doubl
       trial(b0, b1, b2, keep);
     }
     if (best_keep) blocks_pass(best_keep);
+    // the one-launch step, for meshes whose tables and state vectors fit half the L2
+    const double footprint = (double)m.table_block_bytes + 8.0 * sizeof(double) * (m.N + m.nv);
+    if (footprint <= l2 / 2) {
+      try {
+        set_persistent(m, true);
+        use_persistent = faster();
+      } catch (const Error&) {  // no cooperative launch: keep the launches
+      }
+      m.persistent = false;
+    }
+    // The patches; runs too short for them say nothing about longer ones, which keep what they had.
+    if (m.patches.runs && m.use_graph && patches_take(m, steps)) {
+      m.use_patches = true;
+      use_patches = faster();
+      use_persistent = use_persistent && !use_patches;
+    }
   } catch (...) {
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     m.persistent = false;
+    m.use_patches = had_patches;
     throw;
   }
-  // the one-launch step, for meshes whose tables and state vectors fit half the L2
-  bool use_persistent = false;
-  const double footprint = (double)m.table_block_bytes + 8.0 * sizeof(double) * (m.N + m.nv);
-  if (footprint <= l2 / 2) {
-    try {
-      const bool was = m.persistent;
-      set_persistent(m, true);
-      const double before = best_t;
-      trial(best[0], best[1], best[2], best_keep);  // the blocks do not apply to it; best_t moves if faster
-      use_persistent = best_t < before;
-      m.persistent = was;
-    } catch (const Error&) {
-      m.persistent = false;  // no cooperative launch: keep the launches
-    }
-  }
-  // the patches
-  bool use_patches = false;
-  if (m.patches.runs && m.use_graph) {
-    m.use_patches = true;
-    const double before = best_t;
-    trial(best[0], best[1], best[2], best_keep);  // the blocks and the prefix do not apply to them
-    use_patches = best_t < before;
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  m.persistent = use_persistent && !use_patches;
+  m.persistent = use_persistent;
   m.use_patches = use_patches;
   for (int p = 0; p < 3; ++p) m.block[p] = best[p];
   m.l2_keep_bytes = best_keep;
@@ -1308,8 +1328,7 @@ int trisk_autotune(TriskModel* model, double* y, double dt, int32_t steps, doubl
     cudaGraphExecDestroy(m.graph);
     m.graph = nullptr;
   }
-  CUDA_CHECK(cudaMemsetAsync(m.flag, 0, sizeof(int), m.stream));
-  CUDA_CHECK(cudaStreamSynchronize(m.stream));
+  take_marks(m);  // the trials'
   if (best_ms) *best_ms = best_t / steps;
   TRISK_API_END
 }

@@ -229,8 +229,8 @@ int trisk_model_info(TriskModel* model, int32_t* pv_mode, int32_t block[3], doub
  * table prefixes of 8..64 MB (trisk_model_set_l2_residency, no window) with the best blocks,
  * then the blocks again with the best prefix, then (for meshes whose tables and vectors fit
  * half the L2) the one-launch step of trisk_model_set_persistent and (for meshes whose tables
- * fit the SMs' shared memory) the patches, and keeps the fastest in the model; best_ms gets
- * its time per step. */
+ * fit the SMs' shared memory, if runs of `steps` steps take it) the run from shared memory, and
+ * keeps the fastest in the model; best_ms gets its time per step. */
 int trisk_autotune(TriskModel* model, double* y_device, double dt, int32_t steps, double* best_ms);
 /* Sets the threads per block of the three phases (vertex, flux, tend), each a multiple of 32
  * in [64, 256], as an autotuner result found earlier (no reference counterpart). RK4 steps

@@ -462,3 +462,18 @@ def test_timeout_leaves_no_mark_for_the_next_call(require_gpu):
     assert err.value.status == 5
     d.rk4_step(y, dt, d.tendency, d.RK4Cache(y), m, nsteps=9)
     assert np.isfinite(y).all()
+
+
+def test_autotune_of_short_runs_leaves_longer_ones_their_patches(require_gpu):
+    """Four steps of hexagon 3 run as launches, so an autotune of them has no trial of the patches
+    and no say in runs of eight, which are one launch before and after it."""
+    import torch
+    g = trisk_grid(3)
+    si = w.si_parameters()
+    m = d.TRiSKShallowWater(g, **si)
+    dt = w.courant_dt(g, 0.1)
+    y = torch.from_numpy(w.synthetic_state(g, seed=6)).cuda()
+    assert m.autotune(y, dt, 4) > 0
+    before = m.launch_count()
+    d.rk4_step(y, dt, d.tendency, d.RK4Cache(y), m, nsteps=8)
+    assert m.launch_count() - before <= 3
