@@ -136,6 +136,7 @@ def _load():
         "trisk_mpas_stream": (C.c_int, [_p, C.POINTER(_p)]),
         "trisk_mpas_synchronize": (C.c_int, [_p]),
         "trisk_mpas_launch_count": (_i64, [_p]),
+        "trisk_mpas_levels_per_thread": (_i32, [_p]),
         "trisk_icosahedral_mesh": (C.c_int, [_i32, _i32, _f64, _p, _p]),
         "trisk_lloyd": (C.c_int, [_p, _i64, _p, _i64, _i32, _i32, C.POINTER(_i32)]),
         "trisk_mesh_destroy": (None, [_p]),

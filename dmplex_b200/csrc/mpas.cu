@@ -660,6 +660,8 @@ int trisk_mpas_synchronize(TriskMpas* ops) {
   TRISK_API_END
 }
 
+int32_t trisk_mpas_levels_per_thread(TriskMpas* ops) { return ops ? ops->lpt : -1; }
+
 int64_t trisk_mpas_launch_count(TriskMpas* ops) { return ops ? ops->launches : -1; }
 
 }  // extern "C"

@@ -258,7 +258,7 @@ class MPASOperators:
         self._h = h
         self.nc, self.ne, self.nv, self.nlev = t["nc"], t["ne"], t["nv"], t["nlev"]
         self.vertex_kinetic = bool(s.vertex_kinetic)
-        self.levels_per_thread = int(levels_per_thread) or 8
+        self.levels_per_thread = int(lib.trisk_mpas_levels_per_thread(h))
 
     def __del__(self):
         if getattr(self, "_h", None):

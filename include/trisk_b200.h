@@ -371,6 +371,8 @@ int trisk_mpas_slow_tendencies_async(TriskMpas* ops, const TriskMpasFields* fiel
 int trisk_mpas_stream(TriskMpas* ops, void** stream);
 int trisk_mpas_synchronize(TriskMpas* ops);
 int64_t trisk_mpas_launch_count(TriskMpas* ops);
+/* The levels each thread walks: as given to trisk_mpas_create, or what 0 chose. */
+int32_t trisk_mpas_levels_per_thread(TriskMpas* ops);
 
 /* ---- one rank's part of a distributed model -------------------------------------------
  * Replaces TRiSKShallowWater(grid; comm, part)     src/FiniteVolumes/TRiSKShallowWater.jl:121-168

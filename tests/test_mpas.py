@@ -188,6 +188,16 @@ def test_gpu_without_pressure_is_bitwise(require_gpu):
 
 
 @pytest.mark.gpu
+def test_gpu_reports_the_levels_per_thread_it_runs(require_gpu):
+    """The default is 8 levels a thread, fewer on meshes too small for four blocks an SM (2 at the
+    least); a size that was asked for is kept."""
+    v = mpas.vertical_grid(30, 30000.0, stretch=3)
+    small, large = mpas.mpas_tables(hex_grid(3), v), mpas.mpas_tables(hex_grid(6), v)
+    assert [mpas.MPASOperators(small, levels_per_thread=n).levels_per_thread for n in (0, 1, 16)] == [2, 1, 16]
+    assert mpas.MPASOperators(large).levels_per_thread == 8
+
+
+@pytest.mark.gpu
 def test_gpu_argument_errors(require_gpu):
     import torch
     g = hex_grid(2)
