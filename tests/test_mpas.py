@@ -160,11 +160,7 @@ def _gpu_case(cfg, lpt, nl=10, n=4, pressure=1.0, seed=3):
     return t, ref, got, ops
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("cfg", CONFIGS, ids=["iap", "trisk-vi", "advective"])
-@pytest.mark.parametrize("lpt", [8, 1, 16])
-def test_gpu_matches_oracle(require_gpu, cfg, lpt):
-    t, ref, got, ops = _gpu_case(cfg, lpt)
+def _assert_matches(t, ref, got, ops):
     exact = ["theta", "K", "qv", "zetav", "rhov", "qe", "rhoe", "Fs", "tw"]
     if t["vertical"] > 0:
         exact.append("eta")
@@ -177,6 +173,22 @@ def test_gpu_matches_oracle(require_gpu, cfg, lpt):
     rel = np.linalg.norm(got["tvn"] - ref["tvn"]) / np.linalg.norm(ref["tvn"])
     assert rel <= 1e-12
     assert ops.launch_count() == 5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cfg", CONFIGS, ids=["iap", "trisk-vi", "advective"])
+@pytest.mark.parametrize("lpt", [8, 1, 16])
+def test_gpu_matches_oracle(require_gpu, cfg, lpt):
+    _assert_matches(*_gpu_case(cfg, lpt))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cfg", CONFIGS, ids=["iap", "trisk-vi", "advective"])
+@pytest.mark.parametrize("lpt,nl", [(0, 10), (2, 11), (4, 10), (4, 11)])
+def test_gpu_shorter_runs_match_oracle(require_gpu, cfg, lpt, nl):
+    """The runs of levels that meshes too small to fill the device get (0 picks 2 on hexagon 4), with
+    whole runs and with each size of remainder at the top."""
+    _assert_matches(*_gpu_case(cfg, lpt, nl=nl))
 
 
 @pytest.mark.gpu
