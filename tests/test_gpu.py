@@ -336,8 +336,8 @@ def test_config_level7_gassmann_vertex(require_gpu):
                                              (4, "trisk", "mixed", False), (5, "gassmann", "mixed", True)])
 def test_patches_bitwise(require_gpu, n, pv, ke, reorder):
     """The patches (whole tendencies, and RK4 runs from hexagon 4 or of eight steps, from shared
-    memory) against the oracle and the three-launch tendency, bit for bit: the smallest meshes (patches
-    of four cells, a single block), numberings that are not compact, and a run of one launch."""
+    memory) against the oracle, bit for bit, and RK4 steps of the three-launch phases beside them: the
+    smallest meshes (patches of four cells), numberings that are not compact, and a run of one launch."""
     import torch
     from oracle.oracle import Oracle
     si = w.si_parameters()
@@ -477,3 +477,41 @@ def test_autotune_of_short_runs_leaves_longer_ones_their_patches(require_gpu):
     before = m.launch_count()
     d.rk4_step(y, dt, d.tendency, d.RK4Cache(y), m, nsteps=8)
     assert m.launch_count() - before <= 3
+
+
+@pytest.mark.parametrize("reorder", [True, False])
+@pytest.mark.parametrize("pv,ke", SCHEMES)
+def test_three_launch_tendency_bitwise(require_gpu, pv, ke, reorder):
+    """A tendency of the three phase launches (hexagon 6: smaller meshes take theirs from shared
+    memory) against the oracle, bit for bit."""
+    from oracle.oracle import Oracle
+    si = w.si_parameters()
+    g = trisk_grid(6)
+    m = d.TRiSKShallowWater(g, pv_flux=pv, kinetic_energy=ke, reorder=reorder, **si)
+    y = w.synthetic_state(g, seed=6)
+    dy = np.zeros_like(y)
+    before = m.launch_count()
+    d.tendency(dy, y, m)
+    assert m.launch_count() - before == 3 + 2 * reorder  # and the numbering in and out
+    assert np.array_equal(dy, Oracle(tables(6, pv, ke, False, None, **si), threads=4).tendency(y))
+
+
+def test_patches_with_an_explicit_pv_table_bitwise(require_gpu):
+    """RK4 steps from shared memory with a Gassmann PV table that the kernel cannot derive from the
+    flux edges."""
+    from oracle.oracle import Oracle
+    g = trisk_grid(4, True)
+    t = dict(tables(4, "gassmann", "vertex", True))
+    perm = np.arange(12)
+    perm[[0, 1, 6, 7]] = [1, 0, 7, 6]
+    for name in ("g_edges", "g_pv_edges", "g_weights"):
+        t[name] = np.ascontiguousarray(t[name][:, perm])
+    m = d.TRiSKShallowWater.from_coefficients(t, grid=g, pv_flux="gassmann", kinetic_energy="vertex")
+    assert m.info()["pv_mode"] == 1
+    y = perturbed_tc2(g)
+    ref = y.copy()
+    before = m.launch_count()
+    d.rk4_step(y, 0.01, d.tendency, d.RK4Cache(y), m, nsteps=5)
+    assert m.launch_count() - before <= 3
+    Oracle(t).rk4_step(ref, 0.01, 5)
+    assert np.array_equal(y, ref)
