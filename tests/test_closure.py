@@ -82,9 +82,9 @@ def test_forward_and_gradients_match_oracle(require_gpu, n):
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [31, 129, 38017])
 def test_biases_and_ragged_rows_match_oracle(require_gpu, n):
-    """Biases of the size of the pre-activations (three BF16 terms each in the kernels, so exact) at
-    row counts that leave part of a tile and, at the largest, one more tile for some CTAs; the
-    tolerances of the test above."""
+    """Biases of the size of the pre-activations (columns of the tensor-core operands in the kernels)
+    at row counts that leave part of a tile and, at the largest, one more tile for some CTAs; the
+    tolerances of the test above. test_biases_reach_the_network_whole is the one of their last bits."""
     import torch
     import dmplex_b200.closure as cl
     X, T = _data(n, n + 1)
@@ -104,6 +104,72 @@ def test_biases_and_ragged_rows_match_oracle(require_gpu, n):
     gb, gob = _blocks(g), _blocks(go)
     for name, _ in co.SHAPES:
         assert _rel(gb[name], gob[name]) <= 2e-2, name
+
+
+def _cancelling_bias(layer):
+    """Parameters and a row whose pre-activations in one layer are -64.125 + (64.125 + k 2^-17): the
+    bias's first BF16 term cancels 64, its second 0.125, and what is left is its third."""
+    p = {name: np.zeros(shape) for name, shape in co.SHAPES}
+    k = 8.0 * (1 + np.arange(co.NH) % 6)
+    x = np.zeros((1, co.NIN))
+    x[0, :2] = 1
+    p[layer] = 64.125 + k * 2.0 ** -17
+    if layer == "b1":
+        p["W1"][:, 0], p["W1"][:, 1] = -64, -0.125
+        p["W2"] = 1024.0 * np.eye(co.NH)
+    else:
+        p["W1"][:2, 0] = 64  # gelu(64) = 64
+        p["W2"][:, 0], p["W2"][:, 1] = -1, -2.0 ** -9
+    p["W3"][0], p["W3"][1] = 1, -0.5
+    return co.pack(p), x
+
+
+@pytest.mark.parametrize("layer", ["b1", "b2"])
+def test_cancelling_bias_needs_all_three_terms(layer):
+    """The case below on the CPU: a bias short of its second or third term is far outside the
+    tolerance."""
+    p, x = _cancelling_bias(layer)
+    full = co.forward(p, x)[0]
+    q = co.unpack(p)
+    one = co.bf16(q[layer])
+    for short in (one, one + co.bf16(q[layer] - one)):
+        assert _rel(co.forward(co.pack({**q, layer: short}), x)[0], full) > 0.5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layer", ["b1", "b2"])
+def test_biases_reach_the_network_whole(require_gpu, layer):
+    """A bias is exact in the kernels: where all but its last bits cancel, those decide the output.
+    Tolerance: one BF16 rounding either way in each hidden layer (2^-8 each), all terms of a sign."""
+    import torch
+    import dmplex_b200.closure as cl
+    p, x = _cancelling_bias(layer)
+    X = np.repeat(x, 130, axis=0)
+    Xd = torch.from_numpy(X.astype(np.float32)).to(torch.bfloat16).cuda().contiguous()
+    Y = cl.ClosureMLP(p.astype(np.float32)).forward(Xd).cpu().numpy()
+    assert _rel(Y, co.forward(p, X)[0]) <= 1e-2
+
+
+@pytest.mark.gpu
+def test_output_gradient_reaches_dw3_whole(require_gpu):
+    """dY is exact in dW3 = H2^T dY: with H2 = 64 everywhere and rows whose dY cancel but for its
+    last bits (1 + 2^-10 + 2^-20 against 1 + 2^-10, its three BF16 terms), those are the sum, exactly."""
+    import torch
+    import dmplex_b200.closure as cl
+    n = 256
+    p = {name: np.zeros(shape) for name, shape in co.SHAPES}
+    p["b2"][:] = 64
+    p = co.pack(p)
+    T = np.empty((n, co.NOUT))
+    T[0::2] = -(1 + 2.0 ** -10 + 2.0 ** -20)
+    T[1::2] = 1 + 2.0 ** -10
+    X = np.zeros((n, co.NIN))
+    Xd = torch.from_numpy(X.astype(np.float32)).to(torch.bfloat16).cuda().contiguous()
+    Td = torch.from_numpy(T.astype(np.float32)).cuda().contiguous()
+    g, _ = cl.ClosureMLP(p.astype(np.float32)).gradients(Xd, Td)
+    go, _ = co.gradients(p, X, T)
+    assert np.all(_blocks(go)["W3"] == 64 * (n / 2) * 2.0 ** -20 * 2 / n)
+    assert np.array_equal(_blocks(g)["W3"], _blocks(go)["W3"])
 
 
 @pytest.mark.gpu
