@@ -264,10 +264,14 @@ void ensure_graph(TriskModel& m, double dt) {
 }
 
 constexpr int PERSISTENT_BLOCK = 256;
-// Below this many cells (hexagon 3 has 642) runs of fewer steps than PATCH_RUN_STEPS stay with the
-// twelve launches a step that a caller of one step at a time counts; longer runs, and all runs of
-// larger meshes, take the patches. Measured, us a step in runs of 200, launches / patches: hexagon 2
-// 16.5 / 7.6, hexagon 3 18.0 / 8.3, hexagon 4 18.6 / 7.9, hexagon 5 21.9 / 10.5.
+// Below this many cells (hexagon 3 has 642) runs of fewer steps than PATCH_RUN_STEPS keep twelve
+// launches a step, the number trisk_launch_count has always given for them and the tests assert: the
+// count sets this line, not speed. Longer runs, and all runs of larger meshes, take the patches.
+// Measured, us a synchronous call of 1 / 2 / 4 / 7 steps on a device state (TRiSK, cell K), launches
+// against patches: hexagon 2 41 / 60 / 88 / 143 against 41 / 44 / 60 / 81, hexagon 3 50 / 62 / 99 / 157
+// against 41 / 48 / 60 / 89. A step in runs of 200, launches / patches: hexagon 2 16.5 / 7.5, hexagon 3
+// 18.6 / 7.7, hexagon 4 18.7 / 7.9, hexagon 5 20.7 / 10.6 (Gassmann, vertex K: 16.5 / 7.8, 18.6 / 8.1,
+// 20.6 / 7.9, 22.1 / 10.6).
 constexpr int64_t PATCH_RK4_MIN_CELLS = 1024, PATCH_RUN_STEPS = 8;
 
 // All nsteps RK4 steps as one cooperative launch of k_rk4_persistent.
@@ -320,7 +324,11 @@ void gather(TriskModel& m, double* dst, const double* src, const int32_t* idx, i
 
 // Copies of at least this many bytes between pageable host memory and the device go through the
 // model's pinned buffer. The driver copies pageable memory through its own buffer with one thread,
-// about 9 GB/s here; below a few hundred KB that costs less than waking threads does.
+// about 9 GB/s here; for small states that costs less than waking threads does. Measured, us a call
+// of one RK4 step (Gassmann, vertex K) from and to a pageable state of the given KB: the driver's
+// copies / these on 1, 2, 4 and 8 threads: 20 KB 69 / 79, 79, 82, 91; 80 KB 75 / 92, 91, 111, 99;
+// 320 KB 130 / 116, 107, 102, 101; 1280 KB 335 / 284, 182, 173, 166; 5120 KB 990 / 912, 615, 587, 464.
+// Four threads leave a caller of several models some cores.
 constexpr size_t STAGE_MIN_BYTES = 256 * 1024;
 constexpr int STAGE_THREADS = 4, STAGE_PIECES = 4;
 

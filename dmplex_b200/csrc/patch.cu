@@ -409,7 +409,8 @@ void choose_patches(TriskModel& m) {
   CUDA_CHECK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m.device));
   CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m.device));
   // A patch an SM, of at least four cells. On a B200 a patch of 96 cells with its halo takes about
-  // all of an SM's shared memory; hexagon 5 has 69 a patch and takes 92 to 125 KB.
+  // all of an SM's shared memory; hexagon 5 has 69 a patch and takes 92 to 125 KB. (With the tables in
+  // L2 instead larger patches run too, at hexagon 6 a few per cent either way: patch.cuh.)
   if (m.nc > 96 * (int64_t)sms) return;
   const int n = (int)std::max<int64_t>(1, std::min<int64_t>(sms, m.nc / 4));
   if (!build_patches(m, S, n)) {

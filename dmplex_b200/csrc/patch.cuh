@@ -9,13 +9,15 @@
 // gathers from there with 16-bit local indices. Every value is formed by the expressions of
 // kernels.cuh in the same order, so results are the same bit for bit.
 //
-// Measured (wall clock around a synchronous call of 200 steps, us per RK4 step, before / after):
-// hexagon 4 18.6 / 8.3 (TRiSK, cell K), 20.7 / 8.3 (Gassmann, vertex K); hexagon 5 21.5 / 10.4 and
-// 22.4 / 11.0. Of a stage's 2.6 us on hexagon 5 the exchange of the halo takes about 1.5, the three
-// phases 0.4 each: latency of barriers, shared-memory gathers and the FP64 sums. Larger meshes stay
-// with the launches: the tables no longer fit, and with them read from L2 or streamed from HBM in
-// every stage the patches measured 37 to 53 us on hexagon 6 (launches: 37 to 45) and 118 to 208 on
-// hexagon 7 (123 to 148).
+// Measured (wall clock around a synchronous call of 200 steps, us per RK4 step, launches / patches):
+// hexagon 4 18.7 / 7.9 (TRiSK, cell K), 20.6 / 7.9 (Gassmann, vertex K); hexagon 5 20.7 / 10.6 and
+// 22.1 / 10.6. Of a stage's 2.65 us on hexagon 5 the exchange of the halo takes about 1.5, the three
+// phases the rest: latency of barriers, shared-memory gathers and the FP64 sums. Larger meshes stay
+// with the launches, since the tables no longer fit. Hexagon 6 with this kernel reading them from L2,
+// launches / patches by scheme (runs of 100): TRiSK with cell, vertex, mixed K 33.5 / 31.7, 35.2 /
+// 34.7, 35.5 / 34.9; Gassmann 33.2 / 32.0, 33.6 / 32.2, 35.2 / 39.7; Gassmann mean 36.4 / 38.1, 37.2 /
+// 34.5, 37.6 / 43.8: 2 to 7 % faster for six pairs, 5 to 17 % slower for three, which no one rule on
+// the mesh's size separates. On hexagon 7 such forms measured 118 to 208 (launches 123 to 148).
 #pragma once
 #include "kernels.cuh"
 #include "patch.hpp"

@@ -1,15 +1,14 @@
 // Patch decomposition of a model's mesh: whole tendencies and RK4 runs from shared memory, for
-// meshes whose tables fit there (up to about hexagon 5). A patch is a run of consecutive cells of the internal numbering (compact, along the
-// Hilbert curve) with the edges that appear first in them; its halo is every entity its
-// tendency reads, directly or through the vertex and flux values it recomputes. Each patch has
-// one packed block of tables in local 16-bit indices.
+// meshes whose tables fit there (up to about hexagon 5). A patch is a run of consecutive cells of the
+// internal numbering (compact, along the Hilbert curve) with the edges that appear first in them; its
+// halo is every entity its tendency reads, directly or through the vertex and flux values it
+// recomputes. Each patch has one packed block of tables in local 16-bit indices.
 #pragma once
 #include <cstddef>
 #include <cstdint>
 #include <vector>
 
 struct TriskModel;
-
 
 namespace trisk {
 

@@ -235,7 +235,8 @@ int trisk_autotune(TriskModel* model, double* y_device, double dt, int32_t steps
 /* Sets the threads per block of the three phases (vertex, flux, tend), each a multiple of 32
  * in [64, 256], as an autotuner result found earlier (no reference counterpart). RK4 steps
  * then run as launches of those phases, on small meshes too, which otherwise run from the
- * SMs' shared memory in one launch per call (the same numbers bit for bit). */
+ * SMs' shared memory in one launch per call, below 1024 cells from eight steps a call (the same
+ * numbers bit for bit). */
 int trisk_model_set_block(TriskModel* model, const int32_t block[3]);
 /* The one-launch RK4 step (no reference counterpart): on != 0 runs the RK4 steps of
  * trisk_rk4_step(_async) as one cooperative launch whose blocks do the twelve phases of every
@@ -544,7 +545,7 @@ int trisk_closure_gradients(TriskClosure* closure, const void* X, const float* t
 int trisk_closure_adam(TriskClosure* closure, float lr, float beta1, float beta2, float eps);
 int trisk_closure_synchronize(TriskClosure* closure);
 int trisk_closure_stream(TriskClosure* closure, void** stream);
-/* Launch shape of inference: the persistent grid's CTAs per SM (seven on a B200) and the SMs. */
+/* Launch shape of inference: the persistent grid's CTAs per SM (six on a B200) and the SMs. */
 int trisk_closure_info(TriskClosure* closure, int32_t* forward_ctas_per_sm, int32_t* sms);
 /* Test of the bounded tensor-core wait (no reference counterpart): the next inference call of
  * this closure leaves the first tensor-core operation of tile `tile` (rows 128 tile ..) un-issued,
