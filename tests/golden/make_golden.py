@@ -22,14 +22,16 @@ CASES = (("trisk", "cell", 300.0), ("gassmann", "vertex", 300.0), ("gassmann_mea
 LEVEL, SEED = 3, 21
 
 
-def case_data(pv, ke, dt):
+def case_data(pv, ke, dt, y=None):
+    """The case's mesh summary, its state (seeded, unless one is given), tendency and RK4 step."""
     import dmplex_b200 as d
     from dmplex_b200 import workloads as w
     from oracle.oracle import Oracle
     g = d.TRiSKGrid(d.create_hexagon_mesh(LEVEL, centroidal=True))
     si = w.si_parameters()
     o = Oracle(d.model_tables(g, pv_flux=pv, kinetic_energy=ke, **si))
-    y = w.synthetic_state(g, seed=SEED)
+    if y is None:
+        y = w.synthetic_state(g, seed=SEED)
     dy = o.tendency(y)
     y1 = y.copy()
     o.rk4_step(y1, dt, 1)

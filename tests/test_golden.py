@@ -22,11 +22,16 @@ def _golden(pv, ke):
 @pytest.mark.parametrize("pv,ke,dt", CASES)
 def test_oracle_reproduces_golden(pv, ke, dt):
     g = _golden(pv, ke)
-    now = mg.case_data(pv, ke, dt)
+    now = mg.case_data(pv, ke, dt, g["y"].copy())
     assert np.array_equal(now["mesh"][:3], g["mesh"][:3])
     assert np.allclose(now["mesh"][3:], g["mesh"][3:], rtol=1e-14, atol=0)
-    for k in ("y", "dy", "y1"):
+    for k in ("dy", "y1"):
         assert np.array_equal(now[k], g[k]), k
+    # numpy's vectorised sin and cos differ in the last bits with the host's SIMD width, and so does the
+    # seeded state: sums of 80 terms, then differences of neighbours that are a hundredth of them
+    y, ne = mg.case_data(pv, ke, dt)["y"], int(g["mesh"][1])
+    for part in (slice(None, ne), slice(ne, None)):
+        assert np.abs(y[part] - g["y"][part]).max() <= 1e-12 * np.abs(g["y"][part]).max()
 
 
 @pytest.mark.gpu
