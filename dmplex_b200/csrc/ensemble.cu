@@ -528,26 +528,6 @@ struct TriskEnsemble {
 
 namespace {
 
-template <class F>
-void with_modes_e(int pv, int ke, F&& f) {
-  using std::integral_constant;
-  switch (pv * 3 + ke) {
-    case 0: f(integral_constant<int, 0>{}, integral_constant<int, 0>{}); break;
-    case 1: f(integral_constant<int, 0>{}, integral_constant<int, 1>{}); break;
-    case 2: f(integral_constant<int, 0>{}, integral_constant<int, 2>{}); break;
-    case 3: f(integral_constant<int, 1>{}, integral_constant<int, 0>{}); break;
-    case 4: f(integral_constant<int, 1>{}, integral_constant<int, 1>{}); break;
-    case 5: f(integral_constant<int, 1>{}, integral_constant<int, 2>{}); break;
-    case 6: f(integral_constant<int, 2>{}, integral_constant<int, 0>{}); break;
-    case 7: f(integral_constant<int, 2>{}, integral_constant<int, 1>{}); break;
-    case 8: f(integral_constant<int, 2>{}, integral_constant<int, 2>{}); break;
-    case 9: f(integral_constant<int, 3>{}, integral_constant<int, 0>{}); break;
-    case 10: f(integral_constant<int, 3>{}, integral_constant<int, 1>{}); break;
-    case 11: f(integral_constant<int, 3>{}, integral_constant<int, 2>{}); break;
-    default: throw Error(TRISK_ERR_ARGUMENT, "bad scheme");
-  }
-}
-
 // f(R{}) with R the ensemble's storage type.
 template <class F>
 void with_real(const TriskEnsemble& e, F&& f) {
@@ -682,7 +662,7 @@ std::vector<GroupSet> launch_sets(TriskEnsemble& e, unsigned mask, std::vector<s
 // Resident blocks per SM of the three phases for the current block sizes.
 void layout(TriskEnsemble& e) {
   CUDA_CHECK(cudaDeviceGetAttribute(&e.sms, cudaDevAttrMultiProcessorCount, e.device));
-  with_modes_e(e.pv, e.ke, [&](auto pvc, auto kec) {
+  with_modes(e.pv, e.ke, [&](auto pvc, auto kec) {
     constexpr int PV = decltype(pvc)::value, KE = decltype(kec)::value;
     with_real(e, [&](auto r) {
       using R = decltype(r);
@@ -781,7 +761,7 @@ void enqueue_closure(TriskEnsemble& e, const std::vector<int>& set_slices, int s
 void enqueue_ensemble_step(TriskEnsemble& e, unsigned mask) {
   std::vector<std::vector<int>> members;
   const std::vector<GroupSet> sets = launch_sets(e, mask, &members);
-  with_modes_e(e.pv, e.ke, [&](auto pvc, auto kec) {
+  with_modes(e.pv, e.ke, [&](auto pvc, auto kec) {
     constexpr int PV = decltype(pvc)::value, KE = decltype(kec)::value;
     for (int stage = 1; stage <= 4; ++stage) {
       for (size_t k = 0; k < sets.size(); ++k) {
@@ -1440,7 +1420,7 @@ int trisk_ensemble_features(TriskEnsemble* ens, int32_t group, void* X, const do
     const GroupDesc& D = sl.D;
     const int M = D.M;
     const int64_t rows = m.ne * (int64_t)M;
-    with_modes_e(e.pv, e.ke, [&](auto pvc, auto kec) {
+    with_modes(e.pv, e.ke, [&](auto pvc, auto kec) {
       constexpr int PV = decltype(pvc)::value, KE = decltype(kec)::value;
       with_real(e, [&](auto r) {
         using R = decltype(r);
@@ -1482,7 +1462,7 @@ int trisk_ensemble_energy(TriskEnsemble* ens, int32_t group, double* energies) {
     if (sl.group != group) continue;
     const GroupDesc& D = sl.D;
     const int M = D.M;
-    with_modes_e(e.pv, e.ke, [&](auto pvc, auto kec) {
+    with_modes(e.pv, e.ke, [&](auto pvc, auto kec) {
       constexpr int PV = decltype(pvc)::value, KE = decltype(kec)::value;
       with_real(e, [&](auto r) {
         using R = decltype(r);

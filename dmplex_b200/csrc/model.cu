@@ -165,26 +165,6 @@ void launch(TriskModel& m, void (*kernel)(KArgs...), int64_t grid, int block, cu
   m.launches++;
 }
 
-template <class F>
-void with_modes(int pv, int ke, F&& f) {
-  using std::integral_constant;
-  switch (pv * 3 + ke) {
-    case 0: f(integral_constant<int, 0>{}, integral_constant<int, 0>{}); break;
-    case 1: f(integral_constant<int, 0>{}, integral_constant<int, 1>{}); break;
-    case 2: f(integral_constant<int, 0>{}, integral_constant<int, 2>{}); break;
-    case 3: f(integral_constant<int, 1>{}, integral_constant<int, 0>{}); break;
-    case 4: f(integral_constant<int, 1>{}, integral_constant<int, 1>{}); break;
-    case 5: f(integral_constant<int, 1>{}, integral_constant<int, 2>{}); break;
-    case 6: f(integral_constant<int, 2>{}, integral_constant<int, 0>{}); break;
-    case 7: f(integral_constant<int, 2>{}, integral_constant<int, 1>{}); break;
-    case 8: f(integral_constant<int, 2>{}, integral_constant<int, 2>{}); break;
-    case 9: f(integral_constant<int, 3>{}, integral_constant<int, 0>{}); break;
-    case 10: f(integral_constant<int, 3>{}, integral_constant<int, 1>{}); break;
-    case 11: f(integral_constant<int, 3>{}, integral_constant<int, 2>{}); break;
-    default: throw Error(TRISK_ERR_ARGUMENT, "bad scheme");
-  }
-}
-
 // One tendency: three phase launches. ev: optional 6 events (pairs around each launch).
 // With an L2-resident table prefix the kernels' KEEP variants run (per-table L2 policies).
 void enqueue_tendency(TriskModel& m, const DevStage& S, int epi, cudaEvent_t* ev = nullptr) {

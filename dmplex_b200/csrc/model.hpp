@@ -5,6 +5,7 @@
 
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.hpp"
@@ -44,6 +45,27 @@ bool is_kernel_accessible(const void* p, int device);
 // semantics, on every blocking stream), so a caller's device buffer filled or still read on
 // those streams (PyTorch's default stream among them) is safe to use from `stream`.
 void order_after_caller(cudaStream_t stream, cudaEvent_t ev);
+
+// f(PV, KE) as integral constants, for the kernels' template parameters
+template <class F>
+void with_modes(int pv, int ke, F&& f) {
+  using std::integral_constant;
+  switch (pv * 3 + ke) {
+    case 0: f(integral_constant<int, 0>{}, integral_constant<int, 0>{}); break;
+    case 1: f(integral_constant<int, 0>{}, integral_constant<int, 1>{}); break;
+    case 2: f(integral_constant<int, 0>{}, integral_constant<int, 2>{}); break;
+    case 3: f(integral_constant<int, 1>{}, integral_constant<int, 0>{}); break;
+    case 4: f(integral_constant<int, 1>{}, integral_constant<int, 1>{}); break;
+    case 5: f(integral_constant<int, 1>{}, integral_constant<int, 2>{}); break;
+    case 6: f(integral_constant<int, 2>{}, integral_constant<int, 0>{}); break;
+    case 7: f(integral_constant<int, 2>{}, integral_constant<int, 1>{}); break;
+    case 8: f(integral_constant<int, 2>{}, integral_constant<int, 2>{}); break;
+    case 9: f(integral_constant<int, 3>{}, integral_constant<int, 0>{}); break;
+    case 10: f(integral_constant<int, 3>{}, integral_constant<int, 1>{}); break;
+    case 11: f(integral_constant<int, 3>{}, integral_constant<int, 2>{}); break;
+    default: throw Error(TRISK_ERR_ARGUMENT, "bad scheme");
+  }
+}
 
 // dst[j] = src[idx[j]], j < n, on `stream`
 void launch_gather(cudaStream_t stream, double* dst, const double* src, const int32_t* idx, int64_t n);

@@ -128,24 +128,6 @@ struct Rows {
   }
 };
 
-template <class F>
-void with_modes_p(int pv, int ke, F&& f) {
-  using std::integral_constant;
-  auto k = [&](auto pvc) {
-    switch (ke) {
-      case KE_CELL: f(pvc, integral_constant<int, KE_CELL>{}); break;
-      case KE_VERTEX: f(pvc, integral_constant<int, KE_VERTEX>{}); break;
-      default: f(pvc, integral_constant<int, KE_MIXED>{}); break;
-    }
-  };
-  switch (pv) {
-    case PVM_TRISK: k(integral_constant<int, PVM_TRISK>{}); break;
-    case PVM_GASSMANN: k(integral_constant<int, PVM_GASSMANN>{}); break;
-    case PVM_GASSMANN_MEAN: k(integral_constant<int, PVM_GASSMANN_MEAN>{}); break;
-    default: k(integral_constant<int, PVM_GASSMANN_DERIVED>{}); break;
-  }
-}
-
 }  // namespace
 
 bool build_patches(const TriskModel& m, PatchSet& S, int patches) {
@@ -424,7 +406,7 @@ void choose_patches(TriskModel& m) {
   }
   S.threads = (int)std::min<int64_t>(512, std::max<int64_t>(128, round_up(S.max_items, 32)));
   int occ = 0;
-  with_modes_p(m.pv, m.ke, [&](auto pvc, auto kec) {
+  with_modes(m.pv, m.ke, [&](auto pvc, auto kec) {
     constexpr int PV = decltype(pvc)::value, KE = decltype(kec)::value;
     const void* k = rk4_kernel<PV, KE>();
     allow_smem(k);
@@ -454,7 +436,7 @@ void patch_tendency(TriskModel& m, const double* y, double* dy, const int32_t* m
   A.u_in = y;
   A.dy = dy;
   A.map = map;
-  with_modes_p(m.pv, m.ke, [&](auto pvc, auto kec) {
+  with_modes(m.pv, m.ke, [&](auto pvc, auto kec) {
     constexpr int PV = decltype(pvc)::value, KE = decltype(kec)::value;
     k_patch_tendency<PV, KE><<<S.n, S.threads, S.work_doubles * sizeof(double), m.stream>>>(A);
   });
@@ -472,7 +454,7 @@ void patch_rk4(TriskModel& m, double dt, int64_t nsteps) {
   for (int64_t left = nsteps; left > 0; left -= A.nsteps) {
     A.nsteps = (int)std::min<int64_t>(left, PATCH_STEPS);
     A.base = S.base;
-    with_modes_p(m.pv, m.ke, [&](auto pvc, auto kec) {
+    with_modes(m.pv, m.ke, [&](auto pvc, auto kec) {
       constexpr int PV = decltype(pvc)::value, KE = decltype(kec)::value;
       void* args[] = {&A};
       CUDA_CHECK(cudaLaunchCooperativeKernel(rk4_kernel<PV, KE>(), dim3((unsigned)S.n),
