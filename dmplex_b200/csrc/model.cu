@@ -1408,8 +1408,8 @@ int trisk_model_set_l2_residency(TriskModel* model, int64_t bytes, int32_t windo
 int trisk_model_expire_wait_once(TriskModel* model) {
   TRISK_API_BEGIN
   TriskModel& m = *checked(model);
-  if (!m.patches.runs || m.patches.n < 2)
-    throw Error(TRISK_ERR_UNSUPPORTED, "the model's RK4 runs have no blocks that wait for one another");
+  if (!m.patches.runs || m.patches.n < 2 || m.pv != PVM_TRISK || m.ke != KE_CELL)
+    throw Error(TRISK_ERR_UNSUPPORTED, "the test run is for TRiSK PV fluxes, cell kinetic energy and a small mesh");
   m.patches.expire = true;
   TRISK_API_END
 }

@@ -352,19 +352,20 @@ namespace {
 // Dynamic shared memory of a block with an SM to itself (227 KB less its static part).
 constexpr size_t PATCH_SMEM = 225 * 1024;
 constexpr int PATCH_STEPS = 4096;  // RK4 steps a launch
-// A wait for a neighbour's value takes microseconds; a neighbour may have to wait for an SM that
-// another stream's kernel holds. A run that tests the wait gives up sooner.
-constexpr long long PATCH_WAIT_NS = 10000000000LL, PATCH_TEST_WAIT_NS = 5000000LL;
 
 template <int PV, int KE>
 const void* rk4_kernel() {
   return reinterpret_cast<const void*>(k_patch_rk4<PV, KE>);
 }
 
-void allow_smem(const void* kernel) {
+}  // namespace
+
+void patch_allow_smem(const void* kernel) {
   CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PATCH_SMEM));
   CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
 }
+
+namespace {
 
 PatchParams params(TriskModel& m) {
   PatchSet& S = m.patches;
@@ -409,8 +410,8 @@ void choose_patches(TriskModel& m) {
   with_modes(m.pv, m.ke, [&](auto pvc, auto kec) {
     constexpr int PV = decltype(pvc)::value, KE = decltype(kec)::value;
     const void* k = rk4_kernel<PV, KE>();
-    allow_smem(k);
-    allow_smem(reinterpret_cast<const void*>(k_patch_tendency<PV, KE>));
+    patch_allow_smem(k);
+    patch_allow_smem(reinterpret_cast<const void*>(k_patch_tendency<PV, KE>));
     CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, S.threads, S.smem));
   });
   if ((int64_t)occ * sms < S.n) {
@@ -448,8 +449,7 @@ void patch_rk4(TriskModel& m, double dt, int64_t nsteps) {
   PatchSet& S = m.patches;
   PatchParams A = params(m);
   A.dt = dt;
-  A.wait_ns = S.expire ? PATCH_TEST_WAIT_NS : PATCH_WAIT_NS;
-  A.silent = S.expire ? 0 : -1;
+  const void* expire = S.expire ? patch_expire_kernel() : nullptr;
   S.expire = false;
   for (int64_t left = nsteps; left > 0; left -= A.nsteps) {
     A.nsteps = (int)std::min<int64_t>(left, PATCH_STEPS);
@@ -457,7 +457,7 @@ void patch_rk4(TriskModel& m, double dt, int64_t nsteps) {
     with_modes(m.pv, m.ke, [&](auto pvc, auto kec) {
       constexpr int PV = decltype(pvc)::value, KE = decltype(kec)::value;
       void* args[] = {&A};
-      CUDA_CHECK(cudaLaunchCooperativeKernel(rk4_kernel<PV, KE>(), dim3((unsigned)S.n),
+      CUDA_CHECK(cudaLaunchCooperativeKernel(expire ? expire : rk4_kernel<PV, KE>(), dim3((unsigned)S.n),
                                              dim3((unsigned)S.threads), args, S.smem, m.stream));
     });
     S.base += 4u * (unsigned)A.nsteps;

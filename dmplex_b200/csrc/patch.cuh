@@ -42,8 +42,6 @@ struct PatchParams {
   double dt;
   int nsteps;
   unsigned base;        // the version of the state in y
-  long long wait_ns;    // the longest wait for a neighbour's value
-  int silent;           // a patch that publishes nothing (a test of that wait), or -1
 };
 
 // A patch's table block, in global memory (read past L1) or in shared memory.
@@ -118,9 +116,13 @@ __device__ __forceinline__ void publish(Tagged* p, double x, unsigned version) {
   asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"((b & 0xFFFFFFFFull) | t), "l"((b >> 32) | t)
                : "memory");
 }
-// The value of `version` at p, waited for; false if the wait gave up: after wait_ns (or 2^31 polls,
+// The longest wait for a neighbour's value, which takes microseconds (the neighbour may have to wait
+// for an SM that another stream's kernel holds), and that of a run that tests the wait.
+constexpr long long PATCH_WAIT_NS = 10000000000LL, PATCH_TEST_WAIT_NS = 5000000LL;
+// The value of `version` at p, waited for; false if the wait gave up: after WAIT_NS (or 2^31 polls,
 // which the clock always beats), or when another block's has.
-__device__ __forceinline__ bool receive(const Tagged* p, unsigned version, double& x, int* err, long long wait_ns) {
+template <long long WAIT_NS>
+__device__ __forceinline__ bool receive(const Tagged* p, unsigned version, double& x, int* err) {
   long long start = 0;
   for (unsigned i = 1;; ++i) {
     unsigned long long lo, hi;
@@ -132,7 +134,7 @@ __device__ __forceinline__ bool receive(const Tagged* p, unsigned version, doubl
     if ((i & 255u) == 0) {
       const long long now = barrier_ns();
       if (start == 0) start = now;
-      if (now - start > wait_ns || *reinterpret_cast<volatile int*>(err) != 0 || i >= (1u << 31)) {
+      if (now - start > WAIT_NS || *reinterpret_cast<volatile int*>(err) != 0 || i >= (1u << 31)) {
         atomicExch(err, 1);
         x = 0.0;
         return false;
@@ -364,12 +366,14 @@ __global__ void __launch_bounds__(512, 2) k_patch_tendency(const PatchParams A) 
 // barrier, flag or fence), and blocks may run a stage ahead of one another. The values alternate
 // between two buffers; a patch overwrites version k with k + 2 only after it has received k + 1
 // from every patch that reads it (the halos are symmetric), which those formed after reading k.
-template <int PV, int KE>
-__global__ void __launch_bounds__(512, 1) k_patch_rk4(const PatchParams A) {
+// With EXPIRE (a test of the waits) the first block publishes nothing, so its neighbours give up.
+template <int PV, int KE, bool EXPIRE>
+__device__ __forceinline__ void patch_rk4_run(const PatchParams& A) {
   extern __shared__ __align__(16) double patch_sm[];
   __shared__ PatchDesc D;
   __shared__ int gave_up;
   using W = PatchRows<PV, KE>;
+  constexpr long long WAIT_NS = EXPIRE ? PATCH_TEST_WAIT_NS : PATCH_WAIT_NS;
   const int tid = threadIdx.x, nt = blockDim.x;
   if (tid < (int)(sizeof(PatchDesc) / 4))
     reinterpret_cast<int*>(&D)[tid] = reinterpret_cast<const int*>(A.desc + blockIdx.x)[tid];
@@ -408,7 +412,7 @@ __global__ void __launch_bounds__(512, 1) k_patch_rk4(const PatchParams A) {
         if (step == 0 && stage == EPI_STAGE1)
           x = __ldcg(A.y + g);
         else
-          ok &= receive(A.exchange + (size_t)(version & 1u) * A.N + g, version, x, A.err, A.wait_ns) ? 1 : 0;
+          ok &= receive<WAIT_NS>(A.exchange + (size_t)(version & 1u) * A.N + g, version, x, A.err) ? 1 : 0;
         (edge ? S.u[D.nOE + i] : S.h[D.nOC + i]) = x;
       }
       if (!ok) gave_up = 1;
@@ -457,11 +461,16 @@ __global__ void __launch_bounds__(512, 1) k_patch_rk4(const PatchParams A) {
           akept[j] = stage == EPI_STAGE1 ? kv : akept[j] + 2 * kv;
           next = y + c * kv;
         }
-        if (shared && (int)blockIdx.x != A.silent) publish(out + global(j), next, version + 1u);
+        if (shared && !(EXPIRE && blockIdx.x == 0)) publish(out + global(j), next, version + 1u);
         *slot(j) = next;  // no phase reads the stage state any more
       }
     }
   }
+}
+
+template <int PV, int KE>
+__global__ void __launch_bounds__(512, 1) k_patch_rk4(const PatchParams A) {
+  patch_rk4_run<PV, KE, false>(A);
 }
 
 }  // namespace trisk

@@ -56,6 +56,10 @@ void choose_patches(TriskModel& m);
 void patch_tendency(TriskModel& m, const double* y, double* dy, const int32_t* map);
 // nsteps RK4 steps of the internal state m.y in one cooperative launch.
 void patch_rk4(TriskModel& m, double dt, int64_t nsteps);
+// Lets a kernel have the shared memory of a patch.
+void patch_allow_smem(const void* kernel);
+// The RK4 run whose first block publishes nothing (TRiSK, cell K).
+const void* patch_expire_kernel();
 // The exchanged versions start again, after a run in which a wait gave up.
 void patch_restart(TriskModel& m);
 

@@ -249,8 +249,8 @@ int trisk_model_get_persistent(TriskModel* model, int32_t* on);
 /* Test of the bounded wait (no reference counterpart): in this model's next RK4 run from shared
  * memory one block hands its neighbours nothing, so their waits run out after a few milliseconds and
  * the run reports TRISK_ERR_TIMEOUT at the next synchronizing call; the state is then unspecified.
- * The model stays usable and later runs are unaffected. TRISK_ERR_UNSUPPORTED for a model without
- * such runs. */
+ * The model stays usable and later runs are unaffected. For models with TRiSK PV fluxes and cell
+ * kinetic energy that have such runs, else TRISK_ERR_UNSUPPORTED. */
 int trisk_model_expire_wait_once(TriskModel* model);
 /* L2 residency of the tables (no reference counterpart; the three-launch phases', which RK4
  * steps use while bytes > 0 is set). The first `bytes` of the model's
