@@ -41,7 +41,7 @@
 // back: 10.3 us for 1000 rows (8 CTAs of one tile), 14.6 for 18944 (148 of one), 22.5 for 37888 (296 of
 // one) and 23.5 for 65536 (296, most of two): past one tile's chain the time goes with the CTAs that
 // add their sums, hardly with the tiles. A step of 65536 rows (sums cleared, kernel, loss read back,
-// Adam) takes 44 us by wall clock from C and 55 from Python; it took 95 with dW3, the output layer and
+// Adam) takes 44 us by wall clock from C and 55 from Python; it took 95 to 104 with dW3, the output layer and
 // the biases on the CUDA cores and every tanh evaluated twice.
 //
 // GELU is the tanh form of Hendrycks and Gimpel (2016), gelu(x) = x/2 (1 + tanh(sqrt(2/pi)
